@@ -32,6 +32,7 @@
 //   order: equal to the reference up to rounding.
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -776,127 +777,412 @@ __global__ void __launch_bounds__(256) k_mpi_advect_4d(const double *__restrict_
   }
 }
 
-// The fused step's 4D pass with R cells per thread at consecutive y (same
-// x, vx, vy).  Block (32 x, 4 rows of R y), blockIdx.z = plane group as in
-// k_mpi_advect_4d.  When the R feet share their x, vx and vy cells and
-// their y cells are consecutive (all but a few per mille of the groups),
-// the group reads each (vx, vy) slab's R + 3 rows of four x values once
-// and applies every cell's own weights from registers: 64 (R + 3) / R
-// loads per cell instead of 256.  Other groups interpolate cell by cell.
-template <int R, bool UK3>
-__global__ void __launch_bounds__(128, R <= 2 ? 3 : 2) k_mpi_advect_4d_rows(const double *__restrict__ c, double *__restrict__ fn,
-                                                           const double *__restrict__ ex,
-                                                           const double *__restrict__ ey, HGrid h, double dt,
-                                                           double *__restrict__ part, double *__restrict__ l2,
-                                                           int *__restrict__ err) {
-  const int ix = blockIdx.x * 32 + threadIdx.x;
-  const int iy0 = (blockIdx.y * blockDim.y + threadIdx.y) * R;
-  const int G = gridDim.z;
-  const long long planes = (long long)h.n[2] * h.n[3];
-  const long long nx = h.n[0];
-  double racc[R], sq = 0.;
-#pragma unroll
-  for (int q = 0; q < R; ++q) racc[q] = 0.;
+// ---------------------------------------------------------------------------
+// The tiled 4D advection.  A CTA owns a tile of W x (4 YG) y x V vx grid
+// points and marches along vy: the coefficients its feet can reach (two more
+// points on each side of x, y and vx, five vy slabs) stay in a ring of six
+// shared-memory slabs, the sixth arriving by cp.async while a step computes.
+// A thread owns four cells at consecutive y: a coefficient row is read from
+// shared memory once for the four of them, 112 loads per cell instead of 256.
+//
+// Geometry of the tiles; vy in nseg segments of Q.
+struct Tile4 {
+  int W, YG, V;          // x extent, groups of four y, vx extent
+  int PX, RY, RV, slab;  // W + 4, 4 YG + 4, V + 4, PX * RY * RV
+  unsigned magic;        // ceil(2^32 / PX): i / PX for i < 2^16
+  int nxt, nyt, nvt, Q, nseg;
+  int nitems;
+};
+constexpr int kTileThreads = 256;
+constexpr int kRing = 6;
+
+// Weight j of the cubic B-spline at fractional offset p, for a j known at
+// run time only: z^3/6 (outer) or 2/3 - z^2 + z^3/2 (inner) with z = p or
+// 1 - p.  EXACT evaluates the reference's sequence and selects.
+template <bool EXACT>
+__device__ __forceinline__ double bspline_j(double p, int j) {
+  if (EXACT) {
+    double e[4];
+    bspline_w<true>(p, e);
+    return j <= 0 ? e[0] : (j == 1 ? e[1] : (j == 2 ? e[2] : e[3]));
+  }
+  const double z = (j == 0 || j == 2) ? 1. - p : p;
+  const double z2 = z * z;
+  return (j == 0 || j == 3) ? z2 * z * (1. / 6.) : fma(z2, fma(.5, z, -1.), 2. / 3.);
+}
+
+// The predictor's x part of a thread (it depends on x and vx only) and y part
+// of a row (y and vy): the 3-point weights of the field there and the first
+// of the three points, relative to the tile's field rows and columns.
+constexpr int kTileX = 6;  // c0[3], x, vx, first column
+constexpr int kTileY = 5;  // c1[3], y, first row
+
+// What bounds it: FP64 (about 350 multiply-adds per cell in the sums and 100
+// in the foot, at 64 per clock and SM) and the shared-memory pipe (112 loads
+// of 8 bytes per cell at 128 bytes per clock and SM) take about the same
+// time.  The sign of the field decides whether a cell's vx (vy) taps start
+// at -2 or -1; where the four cells of a thread disagree, the warp reads one
+// slab more in that dimension and each cell's weight is 0 on the slab that
+// is not its own (EXACT skips it), so the lines where a field component changes sign cost a quarter more
+// there and not a second pass.  Cells whose x or y taps start at different
+// points (only beside the planes vx = 0 and vy = 0) take one sweep each;
+// feet further than one cell away interpolate one by one from global memory.
+// Measured (128^4, a field whose zero lines cross the plane): 16.5 ms against
+// 55 to 58 ms for two cells per thread from L1, whose warps ran both branches
+// wherever the two cells' first taps differed (26 ms where they hardly ever
+// did); FP64 pipe 48%, shared-memory pipe 51%, fixed-latency waits first (two
+// warps per scheduler: 255 registers).  384 threads of 168 registers, with
+// spills: 22.3 ms; sums along x first: 17.4 ms.
+template <bool EXACT, bool MOMENT, int PXC>
+__global__ void __launch_bounds__(kTileThreads, 1)
+    k_mpi_advect_4d_tile(const double *__restrict__ c, double *__restrict__ fn, const double *__restrict__ ex,
+                         const double *__restrict__ ey, HGrid h, Tile4 T, double dt, double *__restrict__ part,
+                         double *__restrict__ l2, int *__restrict__ err) {
+  extern __shared__ __align__(16) double sm[];
+  const int PX = PXC ? PXC : T.PX;
+  const int RY = T.RY, slab = T.slab;
+  const int rows = 4 * T.YG, lines = T.W * T.V;
+  double *fex = sm + kRing * slab, *fey = fex + PX * RY;
+  double *xt = fey + PX * RY;         // [kTileX][lines]
+  double *yt = xt + kTileX * lines;   // [2][kTileY][rows], by the parity of vy
+  int *rowoff = reinterpret_cast<int *>(yt + 2 * kTileY * rows);  // [RV][RY]: a slab's rows in c, -1 past the halo
+  const int tid = threadIdx.x;
+  const int tx = tid % T.W, tr = tid / T.W;
+  const int yg = tr % T.YG, vl = tr / T.YG;
+  const int nx = h.n[0], ny = h.n[1], nvx = h.n[2], nvy = h.n[3];
+  const double hdt = mul(0.5, dt);
+  double sq = 0.;
   bool bad = false;
-  if (ix < h.n[0] && iy0 < h.n[1]) {
-    for (long long p = blockIdx.z; p < planes; p += G) {
-      const int ivx = (int)(p % h.n[2]), ivy = (int)(p / h.n[2]);
-      double g[R][4];
-      bool ok[R];
-      bool fast = true;
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const int iy = iy0 + q;
-        ok[q] = iy < h.n[1] && foot4d<false>(h, ex, ey, ix, iy < h.n[1] ? iy : iy0, ivx, ivy, dt, g[q]);
-        fast &= ok[q];
+  for (int item = blockIdx.x; item < T.nitems; item += gridDim.x) {
+    int r = item;
+    const int x0 = (r % T.nxt) * T.W;
+    r /= T.nxt;
+    const int yt0 = (r % T.nyt) * rows;
+    r /= T.nyt;
+    const int vx0 = (r % T.nvt) * T.V, seg = r / T.nvt, vt = r % T.nvt;
+    const int vy0 = seg * T.Q, vy1 = vy0 + T.Q < nvy ? vy0 + T.Q : nvy;
+    const int x = x0 + tx, y0 = yt0 + 4 * yg, ivx = vx0 + vl;
+    const bool live = vl < T.V && x < nx && y0 < ny && ivx < nvx;
+    __syncthreads();  // the item before has been read
+    // Slab vy of the tile into ring slot `slot`; points past the halo (next
+    // to cells past the grid) are left as they are.
+    for (int i = tid; i < RY * T.RV; i += kTileThreads) {
+      const int v = i / RY, yy = i - v * RY;
+      rowoff[i] = yt0 + yy < ny + 5 && vx0 + v < nvx + 5 ? h.is[1] * yy + h.is[2] * v : -1;
+    }
+    __syncthreads();
+    const int xlim = nx + 5 - x0;
+    auto load_slab = [&](int vy, int slot) {
+      const double *g = c + h.at(x0 - 2, yt0 - 2, vx0 - 2, vy);
+      double *d = sm + slot * slab;
+      for (int i = tid; i < slab; i += kTileThreads) {
+        const int row = PXC ? i / PX : (int)__umulhi((unsigned)i, T.magic);  // i / PX
+        const int xx = i - row * PX, off = rowoff[row];
+        if (off >= 0 && xx < xlim) cp_async8(d + i, g + (off + xx));
       }
-      int ip[R][4];
+    };
+    for (int k = 0; k < 5; ++k) load_slab(vy0 - 2 + k, k);
+    // The field around the tile, periodic.
+    for (int i = tid; i < PX * RY; i += kTileThreads) {
+      const int q = wrapi(x0 - 2 + i % PX, nx) + nx * wrapi(yt0 - 2 + i / PX, ny);
+      fex[i] = __ldg(ex + q);
+      fey[i] = __ldg(ey + q);
+    }
+    // The predictor (foot4d) at (position i of dimension d, velocity v of it).
+    auto predictor = [&](int d, int i, int v, double w[3], double &pos, double &vel) {
+      pos = EXACT ? add(h.minp[d], mul((double)i, h.dx[d])) : h.minp[d] + i * h.dx[d];
+      vel = EXACT ? add(h.minp[d + 2], mul((double)v, h.dx[d + 2])) : h.minp[d + 2] + v * h.dx[d + 2];
+      const double t = EXACT ? mul(h.inv_dx[d], sub(sub(pos, mul(hdt, vel)), h.minp[d]))
+                             : h.inv_dx[d] * (pos - hdt * vel - h.minp[d]);
+      const int ip = (int)fmax(fmin(round(t) - 1., 1e9), -1e9);
+      lag3w<EXACT>(EXACT ? sub(t, (double)ip) : t - ip, w);
+      return ip;
+    };
+    for (int i = tid; i < lines; i += kTileThreads) {
+      double w[3], pos, vel;
+      const int ip = predictor(0, x0 + i % T.W, vx0 + i / T.W, w, pos, vel);
+      xt[i] = w[0];
+      xt[lines + i] = w[1];
+      xt[2 * lines + i] = w[2];
+      xt[3 * lines + i] = pos;
+      xt[4 * lines + i] = vel;
+      xt[5 * lines + i] = (double)(ip - (x0 - 2));
+    }
+    auto y_table = [&](int vy) {
+      if (tid < rows) {
+        double w[3], pos, vel, *t = yt + (vy & 1) * kTileY * rows + tid;
+        const int ip = predictor(1, yt0 + tid, vy, w, pos, vel);
+        t[0] = w[0];
+        t[rows] = w[1];
+        t[2 * rows] = w[2];
+        t[3 * rows] = pos;
+        t[4 * rows] = (double)(ip - (yt0 - 2));
+      }
+    };
+    y_table(vy0);
+    double racc[4] = {0., 0., 0., 0.};
+    int s0 = 0;  // ring slot of slab vy - 2
+    for (int vy = vy0; vy < vy1; ++vy) {
+      cp_async_wait_all();
+      __syncthreads();
+      if (vy + 1 < vy1) {
+        load_slab(vy + 3, s0 == 0 ? kRing - 1 : s0 - 1);
+        y_table(vy + 1);
+      }
+      if (live) {
+        double g[4][4];
+        bool ok[4];
+        // The feet (foot4d, with the field from shared memory: its 3 x 3
+        // points share their rows among the four cells).
+        {
+          const double *xl = xt + vl * T.W + tx;
+          const double *yl = yt + (vy & 1) * kTileY * rows + 4 * yg;
+          const int lx = (int)xl[5 * lines], ly = (int)yl[4 * rows];
+          bool infield = lx >= 0 && lx + 2 < PX && ly >= 0 && ly + 6 <= RY;
 #pragma unroll
-      for (int q = 0; q < R; ++q)
+          for (int q = 1; q < 4; ++q) infield &= yl[4 * rows + q] == yl[4 * rows] + q;
+          if (infield) {
+            const double c0 = xl[0], c1 = xl[lines], c2 = xl[2 * lines];
+            double e1[4] = {0., 0., 0., 0.}, e2[4] = {0., 0., 0., 0.};
+            const double *p1 = fex + ly * PX + lx, *p2 = fey + ly * PX + lx;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) ip[q][j] = (int)floor(g[q][j]);
+            for (int k = 0; k < 6; ++k) {
+              const double a0 = p1[k * PX], a1 = p1[k * PX + 1], a2 = p1[k * PX + 2];
+              const double b0 = p2[k * PX], b1 = p2[k * PX + 1], b2 = p2[k * PX + 2];
+              const double ra = EXACT ? 0. : c0 * a0 + c1 * a1 + c2 * a2;
+              const double rb = EXACT ? 0. : c0 * b0 + c1 * b1 + c2 * b2;
 #pragma unroll
-      for (int q = 1; q < R; ++q)
-        fast &= ip[q][0] == ip[0][0] && ip[q][2] == ip[0][2] && ip[q][3] == ip[0][3] && ip[q][1] == ip[0][1] + q;
-      double val[R];
-      if (fast) {
-        double e0[R][4], e1[R][4], e2[R][4], e3[R][4];
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-          bspline_w<false>(g[q][0] - ip[q][0], e0[q]);
-          bspline_w<false>(g[q][1] - ip[q][1], e1[q]);
-          bspline_w<false>(g[q][2] - ip[q][2], e2[q]);
-          bspline_w<false>(g[q][3] - ip[q][3], e3[q]);
-          val[q] = 0.;
-        }
-        const double *b = c + h.at(ip[0][0] - 1, ip[0][1] - 1, ip[0][2] - 1, ip[0][3] - 1);
-#pragma unroll(UK3 ? 4 : 1)
-        for (int k3 = 0; k3 < 4; ++k3) {
-          // The cells' k3 weights (a select chain when k3 is not a constant).
-          double w3[R];
-#pragma unroll
-          for (int q = 0; q < R; ++q)
-            w3[q] = k3 == 0 ? e3[q][0] : (k3 == 1 ? e3[q][1] : (k3 == 2 ? e3[q][2] : e3[q][3]));
-#pragma unroll
-          for (int k2 = 0; k2 < 4; ++k2) {
-            const double *slab = b + k2 * h.s[2] + k3 * h.s[3];
-            double s2[R];
-#pragma unroll
-            for (int q = 0; q < R; ++q) s2[q] = 0.;
-#pragma unroll
-            for (int r = 0; r < R + 3; ++r) {
-              const double *row = slab + r * h.s[1];
-              const double v0 = __ldg(row), v1 = __ldg(row + 1), v2 = __ldg(row + 2), v3 = __ldg(row + 3);
-#pragma unroll
-              for (int q = 0; q < R; ++q) {
-                const int k1 = r - q;
-                if (k1 >= 0 && k1 < 4) {
-                  const double x = e0[q][0] * v0 + e0[q][1] * v1 + e0[q][2] * v2 + e0[q][3] * v3;
-                  s2[q] = fma(x, e1[q][k1], s2[q]);
+              for (int q = 0; q < 4; ++q) {
+                const int k1 = k - q;
+                if (k1 < 0 || k1 > 2) continue;
+                const double w = yl[k1 * rows + q];
+                if (EXACT) {
+                  const double w0 = mul(c0, w), w1 = mul(c1, w), w2 = mul(c2, w);
+                  e1[q] = add(add(add(e1[q], mul(w0, a0)), mul(w1, a1)), mul(w2, a2));
+                  e2[q] = add(add(add(e2[q], mul(w0, b0)), mul(w1, b1)), mul(w2, b2));
+                } else {
+                  e1[q] = fma(w, ra, e1[q]);
+                  e2[q] = fma(w, rb, e2[q]);
                 }
               }
             }
+            const double xc = xl[3 * lines], vxc = xl[4 * lines];
+            const double vyc = EXACT ? add(h.minp[3], mul((double)vy, h.dx[3])) : h.minp[3] + vy * h.dx[3];
 #pragma unroll
-            for (int q = 0; q < R; ++q) val[q] = fma(s2[q] * e2[q][k2], w3[q], val[q]);
+            for (int q = 0; q < 4; ++q) {
+              const double yc = yl[3 * rows + q];
+              double xs[4];
+              if (EXACT) {
+                xs[0] = sub(xc, mul(dt, sub(vxc, mul(hdt, e1[q]))));
+                xs[1] = sub(yc, mul(dt, sub(vyc, mul(hdt, e2[q]))));
+                xs[2] = fmax(fmin(sub(vxc, mul(dt, e1[q])), h.vtop[2]), h.minp[2]);
+                xs[3] = fmax(fmin(sub(vyc, mul(dt, e2[q])), h.vtop[3]), h.minp[3]);
+              } else {
+                xs[0] = xc - dt * (vxc - hdt * e1[q]);
+                xs[1] = yc - dt * (vyc - hdt * e2[q]);
+                xs[2] = fmax(fmin(vxc - dt * e1[q], h.vtop[2]), h.minp[2]);
+                xs[3] = fmax(fmin(vyc - dt * e2[q], h.vtop[3]), h.minp[3]);
+              }
+              ok[q] = true;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                ok[q] &= !(xs[j] < h.lo[j] || xs[j] > h.hi[j]);
+                g[q][j] = EXACT ? mul(h.inv_dx[j], sub(xs[j], h.minp[j])) : h.inv_dx[j] * (xs[j] - h.minp[j]);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int iy = y0 + q < ny ? y0 + q : ny - 1;
+              ok[q] = foot4d<EXACT>(h, ex, ey, x, iy, ivx, vy, dt, g[q]);
+            }
           }
         }
-      } else {
+        // First cells of the taps relative to the grid point: -1 or 0 in every
+        // dimension.  Bit q of mx, my, m2, m3: 0 for cell q.  b2, b3 = 1 (and
+        // the mask 0) where all cells of the thread say 0.
+        bool fast = true;
+        int b2 = 0, b3 = 0;
+        unsigned mx = 0, my = 0, m2 = 0, m3 = 0;
+        const unsigned all = y0 + 3 < ny ? 15u : (1u << (ny - y0)) - 1u;
+        double out[4] = {0., 0., 0., 0.};
+        double e0[4][4], e1[4][4], e2[4][4], p3[4];
 #pragma unroll
-        for (int q = 0; q < R; ++q) {
-          val[q] = 0.;
-          if (iy0 + q < h.n[1]) {
-            if (ok[q]) val[q] = interp4d<false>(h, c, g[q]);
-            else bad = true;
+        for (int q = 0; q < 4; ++q) {
+          const double f0 = floor(g[q][0]), f1 = floor(g[q][1]), f2 = floor(g[q][2]), f3 = floor(g[q][3]);
+          const int a0 = (int)f0 - x + 1, a1 = (int)f1 - (y0 + q) + 1, a2 = (int)f2 - ivx + 1, a3 = (int)f3 - vy + 1;
+          fast &= (ok[q] && (unsigned)(a0 | a1 | a2 | a3) < 2u) || y0 + q >= ny;
+          mx |= (unsigned)(a0 & 1) << q;
+          my |= (unsigned)(a1 & 1) << q;
+          m2 |= (unsigned)(a2 & 1) << q;
+          m3 |= (unsigned)(a3 & 1) << q;
+          bspline_w<EXACT>(EXACT ? sub(g[q][0], f0) : g[q][0] - f0, e0[q]);
+          bspline_w<EXACT>(EXACT ? sub(g[q][1], f1) : g[q][1] - f1, e1[q]);
+          bspline_w<EXACT>(EXACT ? sub(g[q][2], f2) : g[q][2] - f2, e2[q]);
+          p3[q] = EXACT ? sub(g[q][3], f3) : g[q][3] - f3;
+        }
+        m2 &= all;
+        m3 &= all;
+        if (m2 == all) { b2 = 1; m2 = 0; }
+        if (m3 == all) { b3 = 1; m3 = 0; }
+        if (fast) {
+          const unsigned act = __activemask();
+          const bool five2 = __any_sync(act, m2 != 0), five3 = __any_sync(act, m3 != 0);
+          // Five slabs: every lane reads the same five, all of them loaded.
+          if (five2 && b2) { b2 = 0; m2 = all; }
+          if (five3 && b3) { b3 = 0; m3 = all; }
+          // The sum over the slabs for the cells whose x and y taps start at
+          // (bx, by); MIX: some lane's cells differ in their first slab.
+          auto sweep = [&](auto mixed, unsigned bx, unsigned by, int n3, bool five2, double val[4]) {
+            constexpr bool MIX = decltype(mixed)::value;
+            // First tap: local x = tx + 2 - 1 + (0 or -1) and so on.
+            const double *base = sm + ((vl + b2) * RY + 4 * yg + (int)by) * PX + tx + (int)bx;
+            int slot = s0 + b3;
+            if (slot >= kRing) slot -= kRing;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) val[q] = 0.;
+            // The cells' vx weights on the five slabs (MIX) or the four.
+            double w2[4][MIX ? 5 : 4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const bool later = MIX && ((m2 >> q) & 1);
+#pragma unroll
+              for (int k = 0; k < (MIX ? 5 : 4); ++k)
+                w2[q][k] = later ? (k > 0 ? e2[q][k - 1] : 0.) : (k < 4 ? e2[q][k] : 0.);
+            }
+#pragma unroll 1
+            for (int k3 = 0; k3 < n3; ++k3) {
+              const double *sl = base + slot * slab;
+              if (++slot == kRing) slot = 0;
+              double u[4] = {0., 0., 0., 0.}, w3[4];
+              bool in3[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const int j = MIX ? k3 - (int)((m3 >> q) & 1) : k3;
+                in3[q] = !MIX || (j >= 0 && j < 4);
+                w3[q] = bspline_j<EXACT>(p3[q], j);
+                if (!EXACT && !in3[q]) w3[q] = 0.;
+              }
+#pragma unroll
+              for (int k2 = 0; k2 < (MIX ? 5 : 4); ++k2) {
+                if (MIX && k2 == 4 && !five2) break;
+                const double *row = sl + k2 * RY * PX;
+                // EXACT sums along x first, as the reference does; otherwise y
+                // first: sixteen independent chains of four.
+                double s2[4], t[4][4];
+#pragma unroll
+                for (int k = 0; k < 7; ++k) {
+                  const double v0 = row[k * PX], v1 = row[k * PX + 1], v2 = row[k * PX + 2], v3 = row[k * PX + 3];
+#pragma unroll
+                  for (int q = 0; q < 4; ++q) {
+                    const int k1 = k - q;
+                    if (k1 < 0 || k1 > 3) continue;
+                    if (EXACT) {
+                      const double f3 = add(add(add(mul(e0[q][0], v0), mul(e0[q][1], v1)), mul(e0[q][2], v2)),
+                                            mul(e0[q][3], v3));
+                      s2[q] = k1 == 0 ? mul(f3, e1[q][0]) : add(s2[q], mul(f3, e1[q][k1]));
+                    } else {
+                      const double w = e1[q][k1];
+                      t[q][0] = k1 == 0 ? w * v0 : fma(w, v0, t[q][0]);
+                      t[q][1] = k1 == 0 ? w * v1 : fma(w, v1, t[q][1]);
+                      t[q][2] = k1 == 0 ? w * v2 : fma(w, v2, t[q][2]);
+                      t[q][3] = k1 == 0 ? w * v3 : fma(w, v3, t[q][3]);
+                      if (k1 == 3)
+                        s2[q] = fma(e0[q][1], t[q][1], e0[q][0] * t[q][0]) + fma(e0[q][3], t[q][3], e0[q][2] * t[q][2]);
+                    }
+                  }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  const bool later = MIX && ((m2 >> q) & 1);
+                  const bool in2 = k2 == 0 ? !later : (k2 == 4 ? later : true);
+                  if (EXACT) {
+                    const double v = add(val[q], mul(mul(s2[q], w2[q][k2]), w3[q]));
+                    if (in2 && in3[q]) val[q] = v;
+                  } else {
+                    u[q] = fma(s2[q], w2[q][k2], u[q]);
+                  }
+                }
+              }
+              if (!EXACT) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) val[q] = fma(u[q], w3[q], val[q]);
+              }
+            }
+          };
+          // One sweep per pair of first x and y taps among the thread's
+          // cells: one, except beside the planes vx = 0 and vy = 0.
+          unsigned rem = all;
+          do {
+            const int q0 = rem ? __ffs(rem) - 1 : 0;
+            const unsigned bx = (mx >> q0) & 1, by = (my >> q0) & 1;
+            const unsigned take = rem & (bx ? mx : ~mx) & (by ? my : ~my);
+            rem &= ~take;
+            double val[4];
+            if (five2 || five3) sweep(std::true_type{}, bx, by, five3 ? 5 : 4, five2, val);
+            else sweep(std::false_type{}, bx, by, 4, false, val);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) out[q] = (take >> q) & 1 ? val[q] : out[q];
+          } while (__any_sync(act, rem != 0));
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (y0 + q < ny) {
+              // The foot again: it is rarely needed and not kept.
+              double gq[4];
+              if (foot4d<EXACT>(h, ex, ey, x, y0 + q, ivx, vy, dt, gq)) out[q] = interp4d<EXACT>(h, c, gq);
+              else bad = true;
+            }
+          }
+        }
+        double *o = fn + h.at(x, y0, ivx, vy);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (y0 + q < ny) {
+            o[q * h.s[1]] = out[q];
+            if (MOMENT) {
+              racc[q] += out[q];
+              sq = fma(out[q], out[q], sq);
+            }
           }
         }
       }
+      if (++s0 == kRing) s0 = 0;
+    }
+    if (MOMENT) {
+      // Sum over the tile's vx in order; one partial per (vx tile, segment).
+      __syncthreads();
+      const int cells = T.W * rows;
+      if (vl < T.V) {
 #pragma unroll
-      for (int q = 0; q < R; ++q) {
-        if (iy0 + q < h.n[1]) {
-          fn[h.at(ix, iy0 + q, ivx, ivy)] = val[q];
-          racc[q] += val[q];
-          sq = fma(val[q], val[q], sq);
+        for (int q = 0; q < 4; ++q) sm[vl * cells + (4 * yg + q) * T.W + tx] = live ? racc[q] : 0.;
+      }
+      __syncthreads();
+      double *dst = part + (long long)(vt * T.nseg + seg) * nx * ny;
+      for (int i = tid; i < cells; i += kTileThreads) {
+        const int xx = x0 + i % T.W, yy = yt0 + i / T.W;
+        if (xx < nx && yy < ny) {
+          double s = 0.;
+          for (int v = 0; v < T.V; ++v) s += sm[v * cells + i];
+          dst[xx + (long long)nx * yy] = s;
         }
       }
     }
-#pragma unroll
-    for (int q = 0; q < R; ++q)
-      if (iy0 + q < h.n[1]) part[(long long)blockIdx.z * nx * h.n[1] + ix + nx * (iy0 + q)] = racc[q];
   }
   if (bad) atomicOr(err, 2);
-  // Block sum of sq in a fixed order.
-  __shared__ double ws[4];
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  double v = sq;
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if ((tid & 31) == 0) ws[tid >> 5] = v;
-  __syncthreads();
-  if (tid == 0) {
-    double t = 0.;
-    for (int w = 0; w < (int)(blockDim.x * blockDim.y) / 32; ++w) t += ws[w];
-    const long long bl = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
-    l2[2 * bl] = t;
-    l2[2 * bl + 1] = 0.;
+  if (MOMENT) {
+    // Block sum of sq in a fixed order.
+    __shared__ double ws[kTileThreads / 32];
+    double v = sq;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((tid & 31) == 0) ws[tid >> 5] = v;
+    __syncthreads();
+    if (tid == 0) {
+      double t = 0.;
+      for (int w = 0; w < kTileThreads / 32; ++w) t += ws[w];
+      l2[2 * blockIdx.x] = t;
+      l2[2 * blockIdx.x + 1] = 0.;
+    }
   }
 }
 
@@ -1158,7 +1444,8 @@ int launch_advect_4d(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn,
   const dim3 block(32, 8);
   const long long bx = (h.n[0] + 31) / 32, by = (h.n[1] + 7) / 8;
   const long long planes = (long long)h.n[2] * h.n[3];
-  // One resident wave (see launch_advect_4d_rows_r).
+  // One resident wave: every block walks the planes p = z, z + G, ... at the
+  // same pace, so the blocks in flight read neighbouring (vx, vy) slabs.
   int per_sm = 0;
   VLP4D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mpi_advect_4d<EXACT, MOMENT>, 256, 0));
   long long G = ((long long)c->num_sms * (per_sm > 0 ? per_sm : 1)) / (bx * by);
@@ -1178,67 +1465,86 @@ int launch_advect_4d(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn,
   return VLP4D_OK;
 }
 
-template <int R, bool UK3>
-int launch_advect_4d_rows_r(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn, double dt, int *groups,
-                            long long *blocks, cudaStream_t s) {
-  const dim3 block(32, 4);
-  const long long bx = (h.n[0] + 31) / 32, by = (h.n[1] + 4 * R - 1) / (4 * R);
-  const long long planes = (long long)h.n[2] * h.n[3];
-  // One resident wave: every block walks the planes p = z, z + G, ... at
-  // the same pace, so the blocks in flight read neighbouring (vx, vy)
-  // slabs and the coefficients come from DRAM about once.
-  int per_sm = 0;
-  VLP4D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mpi_advect_4d_rows<R, UK3>, 128, 0));
-  long long G = ((long long)c->num_sms * (per_sm > 0 ? per_sm : 1)) / (bx * by);
-  if (G < 1) G = 1;
-  if (G > planes) G = planes;
-  if (G > c->rho_part_groups) G = c->rho_part_groups;
-  if (G * bx * by > c->mpi_part_cap) G = c->mpi_part_cap / (bx * by);
-  if (G < 1) return fail_msg(VLP4D_ERR_UNSUPPORTED, "mpi 4D advection: too many (x, y) blocks for the partials");
-  k_mpi_advect_4d_rows<R, UK3><<<dim3((unsigned)bx, (unsigned)by, (unsigned)G), block, 0, s>>>(
-      c4, fn, c->ex, c->ey, h, dt, c->rho_part, c->mpi_part, c->d_err);
+// The ring, the field around the tile, the predictor's x and y parts.
+size_t tile4_smem(const Tile4 &T) {
+  return sizeof(double) * ((size_t)kRing * T.slab + 2 * (size_t)T.PX * T.RY + (size_t)kTileX * T.W * T.V +
+                           2 * (size_t)kTileY * 4 * T.YG) +
+         sizeof(int) * (size_t)T.RY * T.RV;
+}
+
+// Tiles of k_mpi_advect_4d_tile: x in equal tiles of at most 32, then the
+// (YG, V) with YG * V threads rows of W whose ring fits and which takes the
+// fewest (rounds of tiles over the SMs) x (steps of a segment): a tile past
+// the grid's edge idles, and every segment starts with five slabs and their
+// latency, about two steps' worth.  False: nothing fits (or more partials
+// than the context holds), and the cell-per-thread kernel runs (48 x 44 x 40
+// x 36 in the reference's arithmetic: 0.555 ms against 0.452 for the tiles).
+bool tile4_config(const vlp4d_ctx *c, const HGrid &h, bool moment, Tile4 &T) {
+  const int lim = smem_limit(c) - 1024;
+  const long long nx = h.n[0], ny = h.n[1], nvx = h.n[2], nvy = h.n[3];
+  Tile4 t;
+  t.nxt = (int)((nx + 31) / 32);
+  t.W = (int)((nx + t.nxt - 1) / t.nxt);
+  t.PX = t.W + 4;
+  t.magic = (unsigned)(((1ULL << 32) + t.PX - 1) / t.PX);
+  double best = 0.;
+  for (int yg = 1; yg <= 8; ++yg)
+    for (int v = 1; v <= 16; ++v) {
+      if (t.W * yg * v > kTileThreads) continue;
+      t.YG = yg;
+      t.V = v;
+      t.RY = 4 * yg + 4;
+      t.RV = v + 4;
+      t.slab = t.PX * t.RY * t.RV;
+      if ((long long)tile4_smem(t) > lim) continue;
+      const long long nyt = (ny + 4 * yg - 1) / (4 * yg), nvt = (nvx + v - 1) / v;
+      if (nyt * nvt * t.nxt > (1 << 24)) continue;
+      for (long long nseg = 1; nseg <= nvy && nseg <= 64; ++nseg) {
+        const long long Q = (nvy + nseg - 1) / nseg;
+        if ((nvy + Q - 1) / Q != nseg) continue;
+        if (moment && nvt * nseg > c->rho_part_groups) continue;
+        const long long items = t.nxt * nyt * nvt * nseg;
+        // A step of a tile: its warps share the SM's FP64 pipe on top of the
+        // latency of one warp's own chain.
+        const int warps = (t.W * yg * v + 31) / 32;
+        const double cost = (double)((items + c->num_sms - 1) / c->num_sms) * (Q + 2) * (warps + 8);
+        if (best > 0. && cost >= best) continue;
+        best = cost;
+        T = t;
+        T.nyt = (int)nyt;
+        T.nvt = (int)nvt;
+        T.Q = (int)Q;
+        T.nseg = (int)nseg;
+        T.nitems = (int)items;
+      }
+    }
+  return best > 0.;
+}
+
+template <bool EXACT, bool MOMENT, int PXC>
+int run_advect_4d_tile(vlp4d_ctx *c, const HGrid &h, const Tile4 &T, const double *c4, double *fn, double dt,
+                       long long *blocks, cudaStream_t s) {
+  auto k = k_mpi_advect_4d_tile<EXACT, MOMENT, PXC>;
+  const size_t smem = tile4_smem(T);
+  VLP4D_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = T.nitems < c->num_sms ? T.nitems : c->num_sms;
+  k<<<grid, kTileThreads, smem, s>>>(c4, fn, c->ex, c->ey, h, T, dt, c->rho_part, c->mpi_part, c->d_err);
   VLP4D_LAUNCH_CHECK();
-  *groups = (int)G;
-  *blocks = G * bx * by;
+  if (blocks) *blocks = grid;
   return VLP4D_OK;
 }
 
-// Cells per thread of the fused 4D pass (VLP4D_MPI_ROWS = 1..4 overrides;
-// 1 is the cell-per-thread kernel).
-int mpi_rows() {
-  static int r = [] {
-    const char *e = getenv("VLP4D_MPI_ROWS");
-    const int v = e && *e ? atoi(e) : 2;
-    return v >= 1 && v <= 4 ? v : 2;
-  }();
-  return r;
-}
-
-// Whether the fused 4D pass unrolls its k3 loop (VLP4D_MPI_UNROLL = 0/1;
-// unrolled: more loads in flight, more registers).
-bool mpi_unroll_k3() {
-  static bool u = [] {
-    const char *e = getenv("VLP4D_MPI_UNROLL");
-    return e && *e ? atoi(e) != 0 : true;
-  }();
-  return u;
-}
-
-int launch_advect_4d_fused(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn, double dt, int *groups,
-                           long long *blocks, cudaStream_t s) {
-  const bool u = mpi_unroll_k3();
-  switch (mpi_rows()) {
-    case 2:
-      return u ? launch_advect_4d_rows_r<2, true>(c, h, c4, fn, dt, groups, blocks, s)
-               : launch_advect_4d_rows_r<2, false>(c, h, c4, fn, dt, groups, blocks, s);
-    case 3:
-      return u ? launch_advect_4d_rows_r<3, true>(c, h, c4, fn, dt, groups, blocks, s)
-               : launch_advect_4d_rows_r<3, false>(c, h, c4, fn, dt, groups, blocks, s);
-    case 4:
-      return u ? launch_advect_4d_rows_r<4, true>(c, h, c4, fn, dt, groups, blocks, s)
-               : launch_advect_4d_rows_r<4, false>(c, h, c4, fn, dt, groups, blocks, s);
-    default: return launch_advect_4d<false, true>(c, h, c4, fn, dt, groups, blocks, s);
-  }
+// The 4D advection of the coefficients c4 into fn's grid points, with the
+// moment partials (groups written to *groups) and per-block sums of squares
+// (*blocks pairs in c->mpi_part) when MOMENT.
+template <bool EXACT, bool MOMENT>
+int launch_advect_4d_any(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn, double dt, int *groups,
+                         long long *blocks, cudaStream_t s) {
+  Tile4 T;
+  if (!c->fused || !tile4_config(c, h, MOMENT, T)) return launch_advect_4d<EXACT, MOMENT>(c, h, c4, fn, dt, groups, blocks, s);
+  if (groups) *groups = T.nvt * T.nseg;
+  if (T.PX == 36) return run_advect_4d_tile<EXACT, MOMENT, 36>(c, h, T, c4, fn, dt, blocks, s);
+  return run_advect_4d_tile<EXACT, MOMENT, 0>(c, h, T, c4, fn, dt, blocks, s);
 }
 
 int launch_rho_halo(vlp4d_ctx *c, const HGrid &h, const double *f, cudaStream_t s) {
@@ -1322,7 +1628,7 @@ int vlp4d_mpi_advect_4d(vlp4d_ctx *ctx, void *fn, void *tmp_fn, double dt, void 
   const HGrid h = make_hgrid(ctx);
   cudaStream_t s = (cudaStream_t)stream;
   VLP4D_CUDA_TRY(cudaMemcpyAsync(tmp_fn, fn, sizeof(double) * (size_t)h.total(), cudaMemcpyDeviceToDevice, s));
-  return launch_advect_4d<true, false>(ctx, h, (const double *)tmp_fn, (double *)fn, dt, nullptr, nullptr, s);
+  return launch_advect_4d_any<true, false>(ctx, h, (const double *)tmp_fn, (double *)fn, dt, nullptr, nullptr, s);
 }
 
 int vlp4d_mpi_field(vlp4d_ctx *ctx, const void *fn, void *stream) {
@@ -1361,7 +1667,7 @@ int vlp4d_mpi_step(vlp4d_ctx *ctx, void *fn, void *fnp1, int iter, void *stream)
   if ((rc = launch_vlines<true, false>(ctx, h, f, f, 3, -kH, h.n[2] + 2 * kH, -kH + 1, h.n[2] + kH - 2, s)))
     return rc;
   long long blocks = 0;
-  if ((rc = launch_advect_4d_fused(ctx, h, f, g, dt, &groups, &blocks, s))) return rc;
+  if ((rc = launch_advect_4d_any<false, true>(ctx, h, f, g, dt, &groups, &blocks, s))) return rc;
   if ((rc = launch_rho_finish(ctx, groups, s))) return rc;
   if ((rc = launch_field_poisson(ctx, s))) return rc;
   if ((rc = launch_diags(ctx, iter, s))) return rc;

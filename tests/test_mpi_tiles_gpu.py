@@ -1,0 +1,70 @@
+"""The tiled vlp4d_mpi 4D advection at the edges of its tiles: x tiles of 32
+and their remainders, groups of four y with one to four cells, partial vx
+tiles and vy segments, and feet on either side of every grid point.
+
+The reference-order entry point is compared bit for bit with the restated
+reference, under fields that leave all first taps within one cell (the tiled
+sums), that change sign from point to point (every mixture of first taps) and
+that push feet several cells away (the cell-by-cell route).  The fused step is
+held to the tolerance of the other fused-step tests (1e-12 of max|f|).
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle.oracle import IC_SLD10, MpiRestatement, interior
+
+pytestmark = pytest.mark.gpu
+
+L, VMAX, DT = 4 * np.pi, 9.0, 0.02
+SHAPES = [(10, 10, 10, 10), (33, 13, 11, 10), (32, 12, 16, 11), (35, 10, 10, 21), (64, 11, 13, 10), (12, 34, 10, 12)]
+
+
+def _dom(pkg, n, nbiter=2):
+    return pkg.Domain(list(n), [0.0, 0.0, -VMAX, -VMAX], [L, L, VMAX, VMAX], DT, nbiter, 10)
+
+
+@pytest.mark.parametrize("cells", [0.0, 0.4, 2.7])
+@pytest.mark.parametrize("n", SHAPES)
+def test_advect_4d_bit_identical(pkg, cuda, n, cells):
+    torch = cuda
+    rest = MpiRestatement(n, (0, 0, -VMAX, -VMAX), (L, L, VMAX, VMAX), DT, 10)
+    rng = np.random.default_rng(sum(n))
+    # The stage takes any coefficients: random ones show every tap.
+    c4 = rng.standard_normal(rest.init_halo(IC_SLD10).shape)
+    # Displacements of up to `cells` cells in vx and vy.
+    scale = cells * (2 * VMAX / max(n[2], n[3])) / DT
+    ex, ey = (scale * rng.uniform(-1, 1, (n[1], n[0])) for _ in range(2))
+    want, err = rest.advect_4d(c4, ex, ey)
+    with pkg.Context(_dom(pkg, n), "f64") as ctx:
+        ctx.ex.copy_(torch.from_numpy(ex).cuda())
+        ctx.ey.copy_(torch.from_numpy(ey).cuda())
+        c = torch.from_numpy(c4).cuda()
+        tmp = ctx.mpi_empty()
+        ctx.mpi_advect_4d(c, tmp, DT)
+        if err:  # the strongest field pushes some x feet of the 64-column grid out of range
+            with pytest.raises(pkg.vlp4d.Vlp4dError) as e:
+                ctx.check()
+            assert e.value.code == pkg.vlp4d.ERR_RANGE
+        else:
+            ctx.check()
+        assert np.array_equal(c.cpu().numpy(), want)
+        assert np.array_equal(tmp.cpu().numpy(), c4)
+
+
+@pytest.mark.parametrize("n", SHAPES)
+def test_fused_step(pkg, cuda, n):
+    torch = cuda
+    rest = MpiRestatement(n, (0, 0, -VMAX, -VMAX), (L, L, VMAX, VMAX), DT, 10)
+    f0 = rest.init_halo(IC_SLD10)
+    fr, diags, _, _ = rest.run_mpi(f0, 2)
+    with pkg.Context(_dom(pkg, n), "f64") as ctx:
+        out = ctx.mpi_run(torch.from_numpy(f0).cuda(), ctx.mpi_empty(), 2)
+        ctx.check()
+        nrj, _ = ctx.diags_read()
+        _, _, l2 = ctx.diags_read_ext()
+        got, want = interior(out.cpu().numpy()), interior(fr)
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+    np.testing.assert_allclose(nrj, diags[:, 0], rtol=0, atol=1e-11)
+    np.testing.assert_allclose(l2, diags[:, 4], rtol=1e-12)
