@@ -68,3 +68,14 @@ def test_fused_step(pkg, cuda, n):
     assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
     np.testing.assert_allclose(nrj, diags[:, 0], rtol=0, atol=1e-11)
     np.testing.assert_allclose(l2, diags[:, 4], rtol=1e-12)
+
+
+@pytest.mark.parametrize("n", [(10, 10, 10, 10), (33, 10, 11, 12), (10, 27, 10, 13), (12, 11, 30, 10)])
+def test_halo_fill_bit_identical(pkg, cuda, n):
+    torch = cuda
+    rest = MpiRestatement(n, (0, 0, -VMAX, -VMAX), (L, L, VMAX, VMAX), DT, 10)
+    f0 = np.random.default_rng(sum(n)).standard_normal(rest.init_halo(IC_SLD10).shape)
+    with pkg.Context(_dom(pkg, n), "f64") as ctx:
+        f = torch.from_numpy(f0).cuda()
+        ctx.mpi_halo_fill(f)
+        assert np.array_equal(f.cpu().numpy(), rest.halo_fill(f0))
