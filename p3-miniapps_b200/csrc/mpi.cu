@@ -264,79 +264,84 @@ __global__ void __launch_bounds__(kHaloThreads) k_mpi_halo(double *__restrict__ 
 //   causal:      t[0] = e[0] + e[1],  t[k] = e[1+k] + alpha t[k-1]
 //   right end:   c[L] = sqrt3 (e[L+1] + sum_{k=0..L-1} alpha^k e[L-k])
 //   anticausal:  c[i] = beta t[i-1] + alpha c[i+1]
-// In place: t[k-1] is stored at e[k] once e[k] has been read.  EXACT runs
-// the reference's order (right-end sum from the original values, products
-// and sums rounded separately); otherwise the right-end sum is accumulated
-// by Horner during the causal pass and products fuse with the sums.
-template <bool EXACT>
+// In place: t[k-1] is stored at e[k] once e[k] has been read; products and
+// sums rounded separately, the right-end sum from the original values.
 __device__ __forceinline__ void spline_line(double *__restrict__ e, long long st, int L, double alpha, double beta,
                                             double sqrt3) {
-  if (EXACT) {
-    double acc = add(e[(long long)(L + 1) * st], e[(long long)L * st]);
-    double ak = alpha;
-    for (int k = 1; k < L; ++k) {
-      acc = add(acc, mul(e[(long long)(L - k) * st], ak));
-      ak = mul(ak, alpha);
-    }
-    double t = add(e[0], e[st]);
-    e[st] = t;
-    for (int k = 1; k < L - 1; ++k) {
-      t = add(e[(long long)(1 + k) * st], mul(alpha, t));
-      e[(long long)(1 + k) * st] = t;
-    }
-    double c = mul(acc, sqrt3);
-    e[(long long)L * st] = c;
-    for (int i = L - 1; i >= 1; --i) {
-      c = add(mul(beta, e[(long long)i * st]), mul(alpha, c));
-      e[(long long)i * st] = c;
-    }
-  } else {
-    // Chunks of 8 positions: the next chunk's values are loaded (in program
-    // order) before the current chunk's results are stored, so the loads
-    // are in flight while the recursion runs.
-    constexpr int C = 8;
-    const double e1 = e[st];
-    double t = e[0] + e1;
-    double hsum = e1;  // Horner: sum_{i=1..L} alpha^(L-i) e[i]
-    e[st] = t;
-    double buf[C], nxt[C];
-#pragma unroll
-    for (int j = 0; j < C; ++j) buf[j] = 2 + j <= L - 1 ? e[(long long)(2 + j) * st] : 0.;
-    for (int i = 2; i <= L - 1; i += C) {
-#pragma unroll
-      for (int j = 0; j < C; ++j) nxt[j] = i + C + j <= L - 1 ? e[(long long)(i + C + j) * st] : 0.;
-#pragma unroll
-      for (int j = 0; j < C; ++j) {
-        if (i + j <= L - 1) {
-          hsum = fma(hsum, alpha, buf[j]);
-          t = fma(alpha, t, buf[j]);
-          e[(long long)(i + j) * st] = t;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < C; ++j) buf[j] = nxt[j];
-    }
-    hsum = fma(hsum, alpha, e[(long long)L * st]);
-    double c = (e[(long long)(L + 1) * st] + hsum) * sqrt3;
-    e[(long long)L * st] = c;
-    // Anticausal: c[i] = beta t[i-1] + alpha c[i+1], the beta products off
-    // the chain.
-#pragma unroll
-    for (int j = 0; j < C; ++j) buf[j] = L - 1 - j >= 1 ? beta * e[(long long)(L - 1 - j) * st] : 0.;
-    for (int i = L - 1; i >= 1; i -= C) {
-#pragma unroll
-      for (int j = 0; j < C; ++j) nxt[j] = i - C - j >= 1 ? beta * e[(long long)(i - C - j) * st] : 0.;
-#pragma unroll
-      for (int j = 0; j < C; ++j) {
-        if (i - j >= 1) {
-          c = fma(alpha, c, buf[j]);
-          e[(long long)(i - j) * st] = c;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < C; ++j) buf[j] = nxt[j];
-    }
+  double acc = add(e[(long long)(L + 1) * st], e[(long long)L * st]);
+  double ak = alpha;
+  for (int k = 1; k < L; ++k) {
+    acc = add(acc, mul(e[(long long)(L - k) * st], ak));
+    ak = mul(ak, alpha);
   }
+  double t = add(e[0], e[st]);
+  e[st] = t;
+  for (int k = 1; k < L - 1; ++k) {
+    t = add(e[(long long)(1 + k) * st], mul(alpha, t));
+    e[(long long)(1 + k) * st] = t;
+  }
+  double c = mul(acc, sqrt3);
+  e[(long long)L * st] = c;
+  for (int i = L - 1; i >= 1; --i) {
+    c = add(mul(beta, e[(long long)i * st]), mul(alpha, c));
+    e[(long long)i * st] = c;
+  }
+}
+
+// The fused step's prefilter splits a line of L = n + 4 points into segments
+// of S consecutive points, each in one thread's registers: a first-order
+// recursion y_k = x_k + alpha y_{k-1} over a segment needs only the last
+// value c of the segment before, y_k(segment) + alpha^(k+1) c, and those
+// follow from the segments' own last values with the factor alpha^S.  Equal
+// to the recursion along the whole line up to rounding; the chain is S + the
+// number of segments instead of 2 L.  Extension included: the points
+// -2, -1, n, n+1 are read as their periodic images, the boundary sums e0, eR
+// (points -3 and n+2) are formed from the line.
+constexpr double kAlpha = 1.7320508075688772 - 2.;  // sqrt(3) - 2
+__host__ __device__ constexpr double alpha_pow(int k) {
+  double r = 1.;
+  for (int i = 0; i < k; ++i) r *= kAlpha;
+  return r;
+}
+// alpha^0 .. alpha^17 as operands from constant memory.
+__constant__ double kAlphaPow[18] = {alpha_pow(0),  alpha_pow(1),  alpha_pow(2),  alpha_pow(3),  alpha_pow(4),
+                                     alpha_pow(5),  alpha_pow(6),  alpha_pow(7),  alpha_pow(8),  alpha_pow(9),
+                                     alpha_pow(10), alpha_pow(11), alpha_pow(12), alpha_pow(13), alpha_pow(14),
+                                     alpha_pow(15), alpha_pow(16), alpha_pow(17)};
+
+// The segments are aligned to the line's right end: position L is the last
+// point of the last one.  Position 0 holds e0 / alpha (the causal pass starts
+// from t_1 = x_1 + e0), positions before it 0.
+template <int S>
+__device__ __forceinline__ void seg_causal(double v[S]) {
+#pragma unroll
+  for (int j = 1; j < S; ++j) v[j] = fma(kAlphaPow[1], v[j - 1], v[j]);
+}
+template <int S>
+__device__ __forceinline__ void seg_causal_carry(double v[S], double c) {
+#pragma unroll
+  for (int j = 0; j < S; ++j) v[j] = fma(kAlphaPow[j + 1], c, v[j]);
+}
+// Between the passes: beta t below position L; at L (the last point of the
+// `last` segment) c[L] = sqrt3 (eR + the right-end sum, which is the causal
+// value without e0's part; aL = alpha^(L-1)).
+template <int S>
+__device__ __forceinline__ void seg_turn(double v[S], bool last, double beta, double sqrt3, double e0, double eR,
+                                         double aL) {
+  const double cL = (eR + fma(-aL, e0, v[S - 1])) * sqrt3;
+#pragma unroll
+  for (int j = 0; j < S; ++j) v[j] *= beta;
+  if (last) v[S - 1] = cL;
+}
+template <int S>
+__device__ __forceinline__ void seg_anticausal(double v[S]) {
+#pragma unroll
+  for (int j = S - 2; j >= 0; --j) v[j] = fma(kAlphaPow[1], v[j + 1], v[j]);
+}
+template <int S>
+__device__ __forceinline__ void seg_anticausal_carry(double v[S], double c) {
+#pragma unroll
+  for (int j = 0; j < S; ++j) v[j] = fma(kAlphaPow[S - j], c, v[j]);
 }
 
 // Cubic B-spline weights at fractional offset w (Advection.hpp:127-144),
@@ -375,18 +380,111 @@ namespace {
 // a thread walking a row and its neighbour walking the next row then hit
 // different banks.
 
-// x lines of every row, then y lines of columns x in [-2, nx+1]
-// (Spline.hpp:128-196: the row update covers all rows, the column update
-// the columns istart..iend).
-template <bool EXACT>
-__device__ void plane_prefilter(double *pl, int P, const HGrid &h) {
-  const int E1 = h.n[1] + 2 * kH, E0 = h.n[0] + 2 * kH;
-  for (int r = threadIdx.x; r < E1; r += blockDim.x)
-    spline_line<EXACT>(pl + (long long)r * P, 1, h.n[0] + 4, h.alpha, h.beta, h.sqrt3);
-  __syncthreads();
-  for (int c = 1 + threadIdx.x; c < E0 - 1; c += blockDim.x)
-    spline_line<EXACT>(pl + c, P, h.n[1] + 4, h.alpha, h.beta, h.sqrt3);
-  __syncthreads();
+// Lines of a plane in shared memory, extended and prefiltered in place: line
+// l (of `lines`) starts at pl + l * ls, position k of it (0 .. n + 5) is st * k
+// further; positions 3 .. n + 2 are given, all are written.  G lanes share a
+// line, S points each (G S >= n + 4).  Lines outside [flo, fhi] are extended
+// only.  aL = alpha^(n + 3).
+template <int S, int G, int ST>
+__device__ __noinline__ void plane_lines(double *pl, int st_, int ls, int n, int lines, int flo, int fhi, double beta,
+                                         double sqrt3, double aL) {
+  const int st = ST ? ST : st_;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  constexpr int kPer = 32 / G;
+  const int g = lane % G, sub = lane / G;
+  const int k0 = n + 5 - (G - g) * S;  // L = n + 4
+  double aw = kAlpha;  // alpha^(g mod 8 + 1): this lane's term of the boundary sums
+  for (int t = 0; t < (g & 7); ++t) aw *= kAlpha;
+  // The image this lane copies: positions 1, 2 <- n+1, n+2; n+3, n+4 <- 3, 4.
+  const int to = g < 2 ? 1 + g : n + 1 + g, from = g < 2 ? n + 1 + g : 1 + g;
+  for (int l0 = warp * kPer; l0 < lines; l0 += nwarps * kPer) {
+    const int l = l0 + sub;
+    const bool on = l < lines;
+    const bool filter = l >= flo && l <= fhi;
+    double *p = pl + (on ? l : lines - 1) * ls;
+    // left: sum_j alpha^j f(n-2-j) (position n+1-j); right: f(1+j) (4+j)
+    double e0 = aw * p[(n - (g & 7)) * st], eR = aw * p[(5 + (g & 7)) * st];
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) {
+      e0 += __shfl_xor_sync(0xffffffffu, e0, d);
+      eR += __shfl_xor_sync(0xffffffffu, eR, d);
+    }
+    if (on && g < 4) p[to * st] = p[from * st];
+    if (on && g == 4) p[0] = filter ? e0 * (1. / kAlpha) : e0;
+    if (on && g == 5) p[(n + 5) * st] = eR;
+    __syncwarp();
+    double v[S];
+    double *q = p + k0 * st;
+#pragma unroll
+    for (int j = 0; j < S; ++j) v[j] = k0 + j >= 0 ? q[j * st] : 0.;
+    seg_causal<S>(v);
+    // The lanes' last values, summed up with alpha^S per lane.
+    double x = v[S - 1], A = alpha_pow(S);
+#pragma unroll
+    for (int d = 1; d < G; d <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, x, d, G);
+      if (g >= d) x = fma(A, y, x);
+      A *= A;
+    }
+    x = __shfl_up_sync(0xffffffffu, x, 1, G);
+    seg_causal_carry<S>(v, g ? x : 0.);
+    seg_turn<S>(v, g == G - 1, beta, sqrt3, e0, eR, aL);
+    seg_anticausal<S>(v);
+    x = v[0];
+    A = alpha_pow(S);
+#pragma unroll
+    for (int d = 1; d < G; d <<= 1) {
+      const double y = __shfl_down_sync(0xffffffffu, x, d, G);
+      if (g + d < G) x = fma(A, y, x);
+      A *= A;
+    }
+    x = __shfl_down_sync(0xffffffffu, x, 1, G);
+    seg_anticausal_carry<S>(v, g < G - 1 ? x : 0.);
+    __syncwarp();  // every lane of the line has read it
+    if (on && filter) {
+#pragma unroll
+      for (int j = 0; j < S; ++j)
+        if (k0 + j >= 1) q[j * st] = v[j];
+      if (g == 0) p[0] = e0;
+    }
+    __syncwarp();
+  }
+}
+
+// The same with one thread per line, for lines too long for 32 segments of 17.
+__device__ __noinline__ void plane_lines_long(double *pl, int st, int ls, int n, int lines, int flo, int fhi,
+                                              double beta, double sqrt3) {
+  for (int l = threadIdx.x; l < lines; l += blockDim.x) {
+    double *p = pl + l * ls;
+    double w = kAlpha, e0 = 0., eR = 0.;
+    for (int j = 1; j <= kMmax; ++j) {
+      e0 = fma(p[(n + 1 - j) * st], w, e0);
+      eR = fma(p[(4 + j) * st], w, eR);
+      w *= kAlpha;
+    }
+    p[0] = e0;
+    p[st] = p[(n + 1) * st];
+    p[2 * st] = p[(n + 2) * st];
+    p[(n + 3) * st] = p[3 * st];
+    p[(n + 4) * st] = p[4 * st];
+    p[(n + 5) * st] = eR;
+    if (l >= flo && l <= fhi) spline_line(p, st, n + 4, kAlpha, beta, sqrt3);
+  }
+}
+
+// S points per lane and G lanes per line for lines of n + 4 points (odd S:
+// the lanes of a line fall on distinct shared-memory banks).
+template <int ST>
+__device__ __forceinline__ void plane_lines_any(double *pl, int st, int ls, int n, int lines, int flo, int fhi,
+                                                double beta, double sqrt3, double aL) {
+  const int L = n + 4;
+  if (L <= 40) plane_lines<5, 8, ST>(pl, st, ls, n, lines, flo, fhi, beta, sqrt3, aL);
+  else if (L <= 72) plane_lines<9, 8, ST>(pl, st, ls, n, lines, flo, fhi, beta, sqrt3, aL);
+  else if (L <= 104) plane_lines<13, 8, ST>(pl, st, ls, n, lines, flo, fhi, beta, sqrt3, aL);
+  else if (L <= 136) plane_lines<17, 8, ST>(pl, st, ls, n, lines, flo, fhi, beta, sqrt3, aL);
+  else if (L <= 272) plane_lines<17, 16, ST>(pl, st, ls, n, lines, flo, fhi, beta, sqrt3, aL);
+  else if (L <= 544) plane_lines<17, 32, ST>(pl, st, ls, n, lines, flo, fhi, beta, sqrt3, aL);
+  else plane_lines_long(pl, st, ls, n, lines, flo, fhi, beta, sqrt3);
 }
 
 // Spline::computeCoeff_xy on every plane of a halo-filled array, in place,
@@ -401,63 +499,15 @@ __global__ void __launch_bounds__(256) k_mpi_spline_xy(double *__restrict__ f, H
       for (int c = threadIdx.x; c < E0; c += blockDim.x) cp_async8(pl + r * P + c, g + (long long)r * E0 + c);
     cp_async_wait_all();
     __syncthreads();
-    // plane_prefilter indexes threads linearly.
     const int tid = threadIdx.y * blockDim.x + threadIdx.x, nt = blockDim.x * blockDim.y;
-    for (int r = tid; r < E1; r += nt) spline_line<true>(pl + (long long)r * P, 1, h.n[0] + 4, h.alpha, h.beta, h.sqrt3);
+    for (int r = tid; r < E1; r += nt) spline_line(pl + (long long)r * P, 1, h.n[0] + 4, h.alpha, h.beta, h.sqrt3);
     __syncthreads();
-    for (int c = 1 + tid; c < E0 - 1; c += nt) spline_line<true>(pl + c, P, h.n[1] + 4, h.alpha, h.beta, h.sqrt3);
+    for (int c = 1 + tid; c < E0 - 1; c += nt) spline_line(pl + c, P, h.n[1] + 4, h.alpha, h.beta, h.sqrt3);
     __syncthreads();
     for (int r = threadIdx.y; r < E1; r += blockDim.y)
       for (int c = threadIdx.x; c < E0; c += blockDim.x) g[(long long)r * E0 + c] = pl[r * P + c];
     __syncthreads();
   }
-}
-
-// The x, y halo of a plane whose interior rows 3..ny+2, columns 3..nx+2 are
-// loaded: x extension of the interior rows, then y extension of every
-// column (a corner then holds the y sum of x sums: the reference's double
-// sum up to rounding).
-__device__ void plane_extend(double *pl, int P, const HGrid &h) {
-  const int nx = h.n[0], ny = h.n[1];
-  const int E0 = nx + 2 * kH;
-  for (int i = threadIdx.x; i < ny * 6; i += blockDim.x) {
-    double *row = pl + (long long)(i / 6 + kH) * P;
-    const int k = i % 6;
-    double v;
-    if (k == 0 || k == 5) {
-      // left: sum_j alpha^j f(nx-2-j) (column nx+1-j); right: f(1+j) (column 4+j)
-      double w = h.alpha, s = 0.;
-      for (int j = 1; j <= kMmax; ++j) {
-        s = fma(row[k == 0 ? nx + 1 - j : 4 + j], w, s);
-        w *= h.alpha;
-      }
-      v = s;
-      row[k == 0 ? 0 : nx + 5] = v;
-    } else {
-      // columns 1, 2 <- nx+1, nx+2 ; nx+3, nx+4 <- 3, 4
-      const int dst = k <= 2 ? k : nx + k;  // k = 3, 4 -> nx+3, nx+4
-      const int src = k <= 2 ? nx + k : k;
-      row[dst] = row[src];
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < E0 * 6; i += blockDim.x) {
-    const int c = i / 6, k = i % 6;
-    double *col = pl + c;
-    if (k == 0 || k == 5) {
-      double w = h.alpha, s = 0.;
-      for (int j = 1; j <= kMmax; ++j) {
-        s = fma(col[(long long)(k == 0 ? ny + 1 - j : 4 + j) * P], w, s);
-        w *= h.alpha;
-      }
-      col[(long long)(k == 0 ? 0 : ny + 5) * P] = s;
-    } else {
-      const int dst = k <= 2 ? k : ny + k;
-      const int src = k <= 2 ? ny + k : k;
-      col[(long long)dst * P] = col[(long long)src * P];
-    }
-  }
-  __syncthreads();
 }
 
 // The fused x/y pass of vlp4d_mpi_step.  Each CTA takes the interior
@@ -468,14 +518,18 @@ __device__ void plane_extend(double *pl, int P, const HGrid &h) {
 // adding it to the thread's moment accumulators, planes in a fixed order.
 // Thread t owns the CPT cells of column t % nx, rows (t / nx) * CPT ..;
 // it walks them with a sliding window of four x sums, so a cell costs
-// about 4 shared-memory loads instead of 16.  The accumulators go to
+// about 4 shared-memory loads instead of 16.  With the prefilter's lines
+// split into segments (plane_lines) the pass takes 2.22 ms at 128^4 against
+// 4.13 with one thread per line (70 of 512 threads at work at 64^2); one
+// 145 KB plane per SM: the load of the plane and the barriers between the
+// phases are exposed (1.9 TB/s).  The accumulators go to
 // part[blockIdx.x][ix + nx*iy] at the end.  A foot outside the spline's
 // range sets bit 2 of *err (the reference stops: "Time step is too
 // large").
 template <int CPT>
 __global__ void __launch_bounds__(512) k_mpi_xy_pass(const double *__restrict__ fn, double *__restrict__ cxy,
-                                                     HGrid h, int P, double dt, double *__restrict__ part,
-                                                     int *__restrict__ err) {
+                                                     HGrid h, int P, double dt, double aLx, double aLy,
+                                                     double *__restrict__ part, int *__restrict__ err) {
   extern __shared__ __align__(16) double pl[];
   const int nx = h.n[0], ny = h.n[1], nvx = h.n[2];
   const int E0 = nx + 2 * kH, E1 = ny + 2 * kH;
@@ -491,16 +545,33 @@ __global__ void __launch_bounds__(512) k_mpi_xy_pass(const double *__restrict__ 
   bool bad = false;
   for (long long p = blockIdx.x; p < planes; p += gridDim.x) {
     const int ivx = (int)(p % nvx), ivy = (int)(p / nvx);
-    const double *src = fn + h.at(0, 0, ivx, ivy);
-    for (int iy = warp; iy < ny; iy += nwarps)
-      for (int ix = lane; ix < nx; ix += 32) cp_async8(pl + (iy + kH) * P + ix + kH, src + (long long)iy * E0 + ix);
+    {
+      const double *src = fn + h.at(0, 0, ivx, ivy) + (long long)warp * E0 + lane;
+      double *d = pl + (warp + kH) * P + kH + lane;
+      for (int iy = warp; iy < ny; iy += nwarps, src += (long long)nwarps * E0, d += nwarps * P) {
+#pragma unroll 4
+        for (int ix = 0; ix < nx; ix += 32)
+          if (ix + lane < nx) cp_async8(d + ix, src + ix);
+      }
+    }
     cp_async_wait_all();
     __syncthreads();
-    plane_extend(pl, P, h);
-    plane_prefilter<false>(pl, P, h);
-    double *dst = cxy + h.at(-kH, -kH, ivx, ivy);
-    for (int r = warp; r < E1; r += nwarps)
-      for (int c = lane; c < E0; c += 32) dst[(long long)r * E0 + c] = pl[r * P + c];
+    // x lines of the grid's rows, then y lines of every column (the first
+    // and last extended only, as the reference's column update leaves them;
+    // the rows above and below come out as the y sums of x lines).
+    plane_lines_any<1>(pl + kH * P, 1, P, nx, ny, 0, ny - 1, h.beta, h.sqrt3, aLx);
+    __syncthreads();
+    plane_lines_any<0>(pl, P, 1, ny, E0, 1, E0 - 2, h.beta, h.sqrt3, aLy);
+    __syncthreads();
+    {
+      double *dst = cxy + h.at(-kH, -kH, ivx, ivy) + (long long)warp * E0 + lane;
+      const double *q = pl + warp * P + lane;
+      for (int r = warp; r < E1; r += nwarps, dst += (long long)nwarps * E0, q += nwarps * P) {
+#pragma unroll 4
+        for (int k = 0; k < E0; k += 32)
+          if (k + lane < E0) dst[k] = q[k];
+      }
+    }
     // 2D advection at the grid points of the plane, from the coefficients.
     // The shift (dt vx, dt vy) is the same for the whole plane: one cell
     // offset and one set of weights per direction (the reference evaluates
@@ -516,21 +587,22 @@ __global__ void __launch_bounds__(512) k_mpi_xy_pass(const double *__restrict__ 
       // x sums of rows iy0 + my - 1 + r (r = 0 .. CPT + 2), a window of four.
       const double *b = pl + (iy0 + my - 1 + kH) * P + (ix + mx - 1 + kH);
       double w0 = 0., w1 = 0., w2 = 0.;
+      auto rows = [&](bool whole) {
 #pragma unroll
-      for (int r = 0; r < CPT + 3; ++r) {
-        double w3 = 0.;
-        if (iy0 + r - 3 < ny) {  // row needed by some cell of the strip
-          const double *row = b + r * P;
-          w3 = ex[0] * row[0] + ex[1] * row[1] + ex[2] * row[2] + ex[3] * row[3];
+        for (int r = 0; r < CPT + 3; ++r) {
+          double w3 = 0.;
+          if (whole || iy0 + r - 3 < ny) {  // row needed by some cell of the strip
+            w3 = ex[0] * b[0] + ex[1] * b[1] + ex[2] * b[2] + ex[3] * b[3];
+            b += P;
+          }
+          if (r >= 3 && (whole || iy0 + r - 3 < ny)) acc[r - 3] += ey[0] * w0 + ey[1] * w1 + ey[2] * w2 + ey[3] * w3;
+          w0 = w1;
+          w1 = w2;
+          w2 = w3;
         }
-        if (r >= 3) {
-          const int j = r - 3;
-          if (iy0 + j < ny) acc[j] += ey[0] * w0 + ey[1] * w1 + ey[2] * w2 + ey[3] * w3;
-        }
-        w0 = w1;
-        w1 = w2;
-        w2 = w3;
-      }
+      };
+      if (iy0 + CPT <= ny) rows(true);
+      else rows(false);
     }
     __syncthreads();
   }
@@ -553,7 +625,7 @@ __global__ void __launch_bounds__(512) k_mpi_xy_pass(const double *__restrict__ 
 // `in` as they are.  Lines with o in [flo, fhi] are prefiltered (the
 // reference's column update skips the outermost layer of the first v
 // dimension, Spline.hpp:164).  All n + 6 positions go to `out`.
-template <bool EXTEND, bool EXACT>
+template <bool EXTEND>
 __global__ void __launch_bounds__(128) k_mpi_vlines(const double *in, double *out, HGrid h,
                                                     int dim, int olo, int no, int flo, int fhi) {
   extern __shared__ __align__(16) double tiles[];
@@ -599,11 +671,84 @@ __global__ void __launch_bounds__(128) k_mpi_vlines(const double *in, double *ou
         col[(n + 4) * 32] = col[4 * 32];
         col[(n + 5) * 32] = sR;
       }
-      if (o >= flo && o <= fhi) spline_line<EXACT>(col, 32, n + 4, h.alpha, h.beta, h.sqrt3);
+      if (o >= flo && o <= fhi) spline_line(col, 32, n + 4, h.alpha, h.beta, h.sqrt3);
       for (int i = 0; i < E; ++i) out[base + (long long)i * sl] = col[i * 32];
     }
     __syncwarp();
   }
+}
+
+// The fused step's v lines: a block takes 32 lines along `dim` at consecutive
+// points of the extended (x, y) plane (contiguous in memory) and one o; warp w
+// holds S consecutive points of its lane's line in registers,
+// read and written straight from and to global memory in whole 256-byte rows,
+// and the segments exchange one value per direction through shared memory.
+// Bound by HBM: 0.78 ms per direction at 128^4, 5.9 TB/s (a lane per line with
+// the tile in shared memory, its chain of 2 x 132 latencies: 1.49 ms).  Every point of the block's lines has been
+// read at the first barrier, so `in` may be `out`.
+template <int S, int NW>
+__global__ void __launch_bounds__(NW * 32) k_mpi_vlines_seg(const double *in, double *out, HGrid h, int dim, int olo,
+                                                            int flo, int fhi, double aL) {
+  __shared__ double edge[NW][32], sum0[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int n = h.n[dim], k0 = n + 5 - (NW - w) * S;  // L = n + 4
+  const long long sl = h.s[dim];
+  const int o = olo + (int)blockIdx.y;
+  const long long i = (long long)blockIdx.x * 32 + lane;
+  const bool live = i < h.s[2];
+  const long long base = i + h.s[dim == 2 ? 3 : 2] * (o + kH);
+  const double *src = in + base;
+  double v[S];
+#pragma unroll
+  for (int j = 0; j < S; ++j) {
+    const int k = k0 + j;
+    const int at = k < 3 ? k + n : (k >= n + 3 ? k - n : k);
+    v[j] = live && k >= 1 ? src[at * sl] : 0.;
+  }
+  // The boundary sums: the left one by the warp that holds position 0 (or
+  // whose first point is position 1), the right one by the last warp.
+  const bool first = k0 <= 1 && k0 + S > 1, last = w == NW - 1;
+  double e0 = 0., eR = 0.;
+  if (first) {
+#pragma unroll
+    for (int j = 1; j <= kMmax; ++j) e0 = fma(alpha_pow(j), !live ? 0. : src[(n + 1 - j) * sl], e0);
+    sum0[lane] = e0;
+  }
+  if (last) {
+#pragma unroll
+    for (int j = 1; j <= kMmax; ++j) eR = fma(alpha_pow(j), !live ? 0. : src[(4 + j) * sl], eR);
+  }
+  const bool filter = o >= flo && o <= fhi;
+  if (filter) {
+    if (first) {
+#pragma unroll
+      for (int j = 0; j < S; ++j)
+        if (k0 + j == 1) v[j] += e0;
+    }
+    seg_causal<S>(v);
+    edge[w][lane] = v[S - 1];
+  }
+  __syncthreads();
+  if (filter) {
+    double c = 0.;
+    for (int q = 0; q < w; ++q) c = fma(alpha_pow(S), c, edge[q][lane]);
+    seg_causal_carry<S>(v, c);
+    seg_turn<S>(v, last, h.beta, h.sqrt3, sum0[lane], eR, aL);
+    seg_anticausal<S>(v);
+    __syncthreads();
+    edge[w][lane] = v[0];
+    __syncthreads();
+    c = 0.;
+    for (int q = NW - 1; q > w; --q) c = fma(alpha_pow(S), c, edge[q][lane]);
+    seg_anticausal_carry<S>(v, c);
+  }
+  if (!live) return;
+  double *dst = out + base;
+#pragma unroll
+  for (int j = 0; j < S; ++j)
+    if (k0 + j >= 1) dst[(k0 + j) * sl] = v[j];
+  if (first) dst[0] = e0;
+  if (last) dst[(n + 5) * sl] = eR;
 }
 
 }  // namespace
@@ -1456,7 +1601,7 @@ int launch_spline_xy_exact(vlp4d_ctx *c, const HGrid &h, double *f, cudaStream_t
 
 // v lines along `dim` for o in [olo, olo + no), prefiltered for o in
 // [flo, fhi].
-template <bool EXTEND, bool EXACT>
+template <bool EXTEND>
 int launch_vlines(vlp4d_ctx *c, const HGrid &h, const double *in, double *out, int dim, int olo, int no, int flo,
                   int fhi, cudaStream_t s) {
   const size_t tile = sizeof(double) * 32 * (size_t)h.e[dim];
@@ -1465,7 +1610,7 @@ int launch_vlines(vlp4d_ctx *c, const HGrid &h, const double *in, double *out, i
   if (warps > 4) warps = 4;
   if (warps < 1) return fail_msg(VLP4D_ERR_UNSUPPORTED, "mpi v lines: a tile does not fit in shared memory");
   const size_t smem = tile * warps;
-  auto k = k_mpi_vlines<EXTEND, EXACT>;
+  auto k = k_mpi_vlines<EXTEND>;
   VLP4D_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
   VLP4D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * warps, smem));
@@ -1478,10 +1623,30 @@ int launch_vlines(vlp4d_ctx *c, const HGrid &h, const double *in, double *out, i
   return VLP4D_OK;
 }
 
+// The fused step's v lines: extended and prefiltered, along dim.
+int launch_vlines_fused(vlp4d_ctx *c, const HGrid &h, const double *in, double *out, int dim, int olo, int no, int flo,
+                        int fhi, cudaStream_t s) {
+  const int L = h.n[dim] + 4;
+  const double aL = std::pow(h.alpha, L - 1);
+  const dim3 grid((unsigned)((h.s[2] + 31) / 32), (unsigned)no);
+#define VLP4D_SEG(S, NW) k_mpi_vlines_seg<S, NW><<<grid, NW * 32, 0, s>>>(in, out, h, dim, olo, flo, fhi, aL)
+  // Longer lines than 32 segments of 17 hold: a lane per line.
+  if (no > 65535 || L > 17 * 32) return launch_vlines<true>(c, h, in, out, dim, olo, no, flo, fhi, s);
+  if (L <= 40) VLP4D_SEG(5, 8);
+  else if (L <= 72) VLP4D_SEG(9, 8);
+  else if (L <= 104) VLP4D_SEG(13, 8);
+  else if (L <= 136) VLP4D_SEG(17, 8);
+  else if (L <= 272) VLP4D_SEG(17, 16);
+  else VLP4D_SEG(17, 32);
+#undef VLP4D_SEG
+  VLP4D_LAUNCH_CHECK();
+  return VLP4D_OK;
+}
+
 int launch_spline_vxvy_exact(vlp4d_ctx *c, const HGrid &h, double *f, cudaStream_t s) {
-  int rc = launch_vlines<false, true>(c, h, f, f, 2, -kH, h.n[3] + 2 * kH, -kH, h.n[3] + kH - 1, s);
+  int rc = launch_vlines<false>(c, h, f, f, 2, -kH, h.n[3] + 2 * kH, -kH, h.n[3] + kH - 1, s);
   if (rc) return rc;
-  return launch_vlines<false, true>(c, h, f, f, 3, -kH + 1, h.n[2] + 4, -kH + 1, h.n[2] + kH - 2, s);
+  return launch_vlines<false>(c, h, f, f, 3, -kH + 1, h.n[2] + 4, -kH + 1, h.n[2] + kH - 2, s);
 }
 
 template <int CPT>
@@ -1496,7 +1661,8 @@ int launch_xy_pass_cpt(vlp4d_ctx *c, const HGrid &h, const double *fn, double *c
   const long long planes = (long long)h.n[2] * h.n[3];
   if (grid > planes) grid = planes;
   if (grid > c->rho_part_groups) grid = c->rho_part_groups;
-  k<<<(unsigned)grid, 512, smem, s>>>(fn, cxy, h, plane_stride(h), dt, c->rho_part, c->d_err);
+  k<<<(unsigned)grid, 512, smem, s>>>(fn, cxy, h, plane_stride(h), dt, std::pow(h.alpha, h.n[0] + 3),
+                                      std::pow(h.alpha, h.n[1] + 3), c->rho_part, c->d_err);
   VLP4D_LAUNCH_CHECK();
   *groups = (int)grid;
   return VLP4D_OK;
@@ -1751,8 +1917,8 @@ int vlp4d_mpi_step(vlp4d_ctx *ctx, void *fn, void *fnp1, int iter, void *stream)
   if ((rc = launch_field_poisson(ctx, s))) return rc;
   // vx lines of the interior vy planes (g -> f), then vy lines of every vx
   // position (in place in f): f holds the 4D coefficients.
-  if ((rc = launch_vlines<true, false>(ctx, h, g, f, 2, 0, h.n[3], 0, h.n[3] - 1, s))) return rc;
-  if ((rc = launch_vlines<true, false>(ctx, h, f, f, 3, -kH, h.n[2] + 2 * kH, -kH + 1, h.n[2] + kH - 2, s)))
+  if ((rc = launch_vlines_fused(ctx, h, g, f, 2, 0, h.n[3], 0, h.n[3] - 1, s))) return rc;
+  if ((rc = launch_vlines_fused(ctx, h, f, f, 3, -kH, h.n[2] + 2 * kH, -kH + 1, h.n[2] + kH - 2, s)))
     return rc;
   long long blocks = 0;
   if ((rc = launch_advect_4d_any<false, true>(ctx, h, f, g, dt, &groups, &blocks, s))) return rc;

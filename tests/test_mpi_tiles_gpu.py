@@ -79,3 +79,39 @@ def test_halo_fill_bit_identical(pkg, cuda, n):
         f = torch.from_numpy(f0).cuda()
         ctx.mpi_halo_fill(f)
         assert np.array_equal(f.cpu().numpy(), rest.halo_fill(f0))
+
+
+LONG = [(72, 10, 10, 10), (10, 102, 10, 10), (140, 11, 10, 10), (10, 280, 10, 10), (10, 10, 75, 10), (10, 10, 10, 120),
+        (11, 10, 150, 10), (10, 10, 10, 300)]
+# Beyond the lines the restated reference holds (512 points).
+LONGEST = [(10, 560, 10, 10), (10, 10, 560, 10)]
+
+
+@pytest.mark.parametrize("n", LONG + LONGEST)
+def test_fused_step_long_lines(pkg, cuda, n):
+    """Every split of the prefilter's lines into segments, in each dimension
+    (the boxes grow with the grid so that no shift exceeds a cell); the longest
+    against the reference-order entry points."""
+    torch = cuda
+    Lx, Ly = (L * max(1.0, n[d] / 60) for d in (0, 1))
+    rest = MpiRestatement(n, (0, 0, -VMAX, -VMAX), (Lx, Ly, VMAX, VMAX), DT, 10)
+    f0 = rest.init_halo(IC_SLD10)
+    dom = pkg.Domain(list(n), [0.0, 0.0, -VMAX, -VMAX], [Lx, Ly, VMAX, VMAX], DT, 2, 10)
+    with pkg.Context(dom, "f64") as ctx:
+        out = ctx.mpi_run(torch.from_numpy(f0).cuda(), ctx.mpi_empty(), 1)
+        ctx.check()
+        got = interior(out.cpu().numpy())
+        if n in LONGEST:
+            half, tmp = torch.from_numpy(f0).cuda(), ctx.mpi_empty()
+            ctx.mpi_halo_fill(half)
+            ctx.mpi_spline_xy(half)
+            new = half.clone()
+            ctx.mpi_advect_2d(half, tmp, 0.5 * DT)
+            ctx.mpi_field(half)
+            ctx.mpi_spline_vxvy(new)
+            ctx.mpi_advect_4d(new, tmp, DT)
+            ctx.check()
+            want = interior(new.cpu().numpy())
+        else:
+            want = interior(rest.run_mpi(f0, 1)[0])
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
