@@ -219,6 +219,11 @@ int vlp4d_ctx_create(const vlp4d_domain *dom, int dtype, vlp4d_ctx **out) {
   long long fused_groups = 2LL * c->num_sms;
   const long long cap = (256LL << 20) / ((long long)sizeof(double) * nxy);
   if (fused_groups > cap) fused_groups = cap;
+  // Small planes: more blocks per SM, as far as 16 MB of partials go.
+  long long small_groups = (16LL << 20) / ((long long)sizeof(double) * nxy);
+  if (small_groups > 8LL * c->num_sms) small_groups = 8LL * c->num_sms;
+  if (small_groups > c->g.nv()) small_groups = c->g.nv();
+  if (fused_groups < small_groups) fused_groups = small_groups;
   c->rho_part_groups = (int)(fused_groups > groups ? fused_groups : groups);
   CTX_ALLOC(c->rho_part, sizeof(double) * nxy * (size_t)c->rho_part_groups);
   CTX_ALLOC(c->d_err, sizeof(int));
@@ -413,6 +418,8 @@ static int advect_xy_impl(vlp4d_ctx *ctx, const void *fn, void *fnp1, double dt,
   rc = launch_advect_xy(ctx, fn, fnp1, tx, ty, true, true, with_rho, s);
   if (rc != VLP4D_ERR_UNSUPPORTED) return rc;
   if ((rc = fused_declined(ctx))) return rc;
+  rc = launch_xy_cols(ctx, fn, fnp1, tx, ty, 6, with_rho, s);
+  if (rc != VLP4D_ERR_UNSUPPORTED) return rc;
   if ((rc = launch_advect_pair_generic(ctx, false, fn, fnp1, tx, ty, s))) return rc;
   return with_rho ? launch_field_rho(ctx, fnp1, s) : VLP4D_OK;
 }

@@ -257,6 +257,15 @@ bool xyxy64_available(const vlp4d_ctx *c);
 int launch_advect_xyxy_tables(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTable *x11,
                               const StencilTable *y11, bool with_rho, cudaStream_t s);
 
+// advect_cols.cu: x/y (6-tap lines, or the composed 11-tap ones with taps =
+// 11; the moment of the result into rho when with_rho) and vx/vy sweeps of
+// any shape and alignment.  VLP4D_ERR_UNSUPPORTED (nothing launched) under
+// VLP4D_KERNELS=generic and for index ranges beyond 32 bits.
+int launch_xy_cols(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTable *tx, const StencilTable *ty, int taps,
+                   bool with_rho, cudaStream_t s);
+int launch_v_cols(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTable *tvx, const StencilTable *tvy,
+                  cudaStream_t s);
+
 // api.cu: one Strang step f_in -> f_out through scratch (diagnostic slot
 // `iter`, none when negative); x/y and vx/vy passes with explicit tables,
 // fused kernels first, generic ones when the fused kernels decline.
