@@ -1297,11 +1297,6 @@ size_t xyxy64_smem(int R, int nx, int stages, int nvx, int nvy) {
 
 }  // namespace
 
-bool xyxy64_available(const vlp4d_ctx *c) {
-  const int nx = c->g.n[0];
-  return c->fused && c->dtype == VLP4D_F64 && nx % 4 == 0 && 32 % (nx / 4) == 0 && env_int("VLP4D_XYXY64", 1) != 0;
-}
-
 namespace {
 
 bool xyxy64_config(const vlp4d_ctx *c, PlaneCfg &cfg) {
@@ -1335,6 +1330,19 @@ bool xyxy64_config(const vlp4d_ctx *c, PlaneCfg &cfg) {
   }
   return false;
 }
+
+}  // namespace
+
+// Chunks of fewer than five rows (ny without such a divisor) sweep ten halo
+// rows each along x: two passes are faster (five steps, 64 x 74 x 48 x 50 in
+// chunks of two: 1.34 ms joined, 1.10 in two passes; 64 x 49 in seven: 0.76 /
+// 0.80).
+bool xyxy64_available(const vlp4d_ctx *c) {
+  PlaneCfg cfg;
+  return c->fused && xyxy64_config(c, cfg) && (cfg.R >= 5 || cfg.R == c->g.n[1]);
+}
+
+namespace {
 
 template <int NX, int RT>
 int run_xyxy64(vlp4d_ctx *c, PlaneArgs args, PlaneCfg &cfg, bool rho, cudaStream_t s) {
@@ -1387,6 +1395,11 @@ int run_xyxy_any(vlp4d_ctx *c, const PlaneArgs &a, PlaneCfg &cfg, bool rho, cuda
 
 }  // namespace
 
+bool xyxy_runs(const vlp4d_ctx *c) {
+  PlaneCfg cfg;
+  return c->fused && xyxy_config(c, cfg);
+}
+
 // Returns VLP4D_ERR_UNSUPPORTED (without launching anything) when the shape
 // or the buffers do not meet the kernel's requirements; the caller then
 // uses the generic kernels.
@@ -1397,6 +1410,15 @@ int launch_advect_xy(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTabl
   if (!do_x && !do_y) return VLP4D_ERR_UNSUPPORTED;
   PlaneCfg cfg;
   if (!plane_config(c, do_x, do_y, cfg)) return VLP4D_ERR_UNSUPPORTED;
+  // Where the column kernel (launch_xy_cols) is faster, decline: chunks of a
+  // few rows (ny without a divisor up to 32: 64 x 74 rows in pairs, x and y,
+  // FP64 107 against 66 us, FP32 66 against 57; chunks of 7 rows: 45.7 / 43.9 and
+  // 27.1 / 37.5), and in FP64 one row per thread outside the in-place form (72 x
+  // 60 in chunks of 30: 168 / 155 us, 80 x 90 in 18: 242 / 154; four rows per
+  // thread, 100 x 100 in 20: 82 / 104).
+  if (!c->fused_only && do_x && do_y &&
+      (cfg.R < 5 && cfg.R < c->g.n[1] || (c->elem == 8 && !cfg.inplace && cfg.rt == 1)))
+    return VLP4D_ERR_UNSUPPORTED;
   const bool moment = with_rho && do_x && do_y;
   PlaneArgs a = plane_args(c, fn, fnp1, cfg, do_y ? 5 : 0);
   if (tx) a.tx = *tx;

@@ -43,8 +43,9 @@ struct VslabArgs {
   // planes and `row0` halo planes on each side), never wrapped.
   int row0, nin;
   int C;      // columns per chunk
-  int Q;      // output vy rows per item (divides nvy)
-  int nseg;   // nvy / Q
+  int rows;   // output vy rows (owned planes)
+  int Q;      // output vy rows per item (the last segment's may be fewer)
+  int nseg;   // ceil(rows / Q)
   long long nitems;
   int stages;
   StencilTable tvx, tvy;
@@ -83,7 +84,7 @@ __device__ __forceinline__ void vx_sweep(const double (&t)[V + 5], const double 
 // warp releases a slot last can refill it without asking anyone.
 struct SlabCursor {
   long long item;
-  int t, cnt, start, cc;
+  int t, cnt, start, cc, q;
 };
 
 template <bool DVY>
@@ -91,12 +92,14 @@ __device__ __forceinline__ void cursor_item(const VslabArgs &a, SlabCursor &c) {
   if (c.item >= a.nitems) return;
   c.cc = (int)(c.item / a.nseg);
   const int sg = (int)(c.item % a.nseg);
+  const int q = a.rows - sg * a.Q;  // the last segment may be shorter
+  c.q = q < a.Q ? q : a.Q;
   if (DVY) {
     const int2 sp = a.span[c.cc];
-    c.cnt = a.Q + (sp.y - sp.x) + 5;
+    c.cnt = c.q + (sp.y - sp.x) + 5;
     c.start = sg * a.Q + sp.x;
   } else {
-    c.cnt = a.Q;
+    c.cnt = c.q;
     c.start = sg * a.Q;
   }
 }
@@ -188,7 +191,7 @@ __global__ void __launch_bounds__(512) k_vslab(const __grid_constant__ CUtensorM
     cur.item = item;
     cur.t = 0;
     cursor_item<DVY>(a, cur);
-    const int cnt = cur.cnt, cc = cur.cc;
+    const int cnt = cur.cnt, cc = cur.cc, nq = cur.q;
     const int sg = (int)(item % a.nseg);
     const long long ixy = (long long)cc * C + col;
     T wvx[6], wvy[6];
@@ -291,7 +294,7 @@ __global__ void __launch_bounds__(512) k_vslab(const __grid_constant__ CUtensorM
         bool emit = true;
         if (DVY) {
           const int e = t - lag0;
-          emit = e >= 0 && e < a.Q;
+          emit = e >= 0 && e < nq;
         }
         if (emit) {
           if constexpr (kF32) {
@@ -410,32 +413,27 @@ bool vslab_config(const vlp4d_ctx *c, bool do_vx, bool do_vy, VslabCfg &cfg) {
   // Q: the vy segment height.  A CTA streams its items one after another,
   // each item Q output rows plus (with a vy sweep) the five halo rows and
   // the chunk's offset spread, about Q + 6 slabs, and about four slab times
-  // of start-up (tables, the pipeline refilling); with one CTA per SM the
-  // pass takes about ceil(items / SMs) * (Q + halo + 4) slab times.  Q
-  // minimises that among the divisors of nvy up to 128 that still give
-  // every SM an item (the smallest Q when none does).  128^4 FP32: Q = 64
-  // (1024 items, 7 per SM); 64^4 FP32: Q = 32 (60.8 -> 47.6 us for vx+vy
-  // against Q = 8).
+  // of start-up (tables, the pipeline refilling); up to 512 threads per SM
+  // run at a time, so the pass takes about ceil(items / slots) * (Q + halo +
+  // 4) slab times.  Q minimises that over the numbers of segments (the last
+  // one may be shorter).
   const long long nchunks = nxy / cfg.C;
+  const long long slots = (long long)c->num_sms * (512 / cfg.threads);
   int Q = env_int("VLP4D_VSLAB_Q", 0);
   if (Q <= 0) {
-    Q = 0;
     long long best = -1;
     const int halo = do_vy ? 6 : 0;
-    for (int q = nvy < 128 ? nvy : 128; q >= 1; --q) {
-      if (nvy % q) continue;
-      const long long items = nchunks * (nvy / q);
-      if (items < c->num_sms && q != 1) continue;
-      const long long cost = (items + c->num_sms - 1) / c->num_sms * (q + halo + 4);
+    for (int nseg = (nvy + 127) / 128; nseg <= nvy; ++nseg) {
+      const int q = (nvy + nseg - 1) / nseg;
+      const long long items = nchunks * ((nvy + q - 1) / q);
+      const long long cost = (items + slots - 1) / slots * (q + halo + 4);
       if (best < 0 || cost < best) {
         best = cost;
         Q = q;
       }
     }
-    if (!Q) Q = 1;
   }
   if (Q > nvy) Q = nvy;
-  while (Q > 1 && nvy % Q) --Q;
   cfg.Q = Q;
   cfg.stages = env_int("VLP4D_VSLAB_STAGES", f32 && both ? 8 : 4);
   if (cfg.stages < 2 || cfg.stages > kMaxStages) return false;
@@ -484,6 +482,16 @@ int launch_advect_vxvy_tables(vlp4d_ctx *c, const void *fn, void *fnp1, const St
   if (!do_vx && !do_vy) return VLP4D_ERR_UNSUPPORTED;
   VslabCfg cfg;
   if (!vslab_config(c, do_vx, do_vy, cfg)) return VLP4D_ERR_UNSUPPORTED;
+  // Where the column kernel (launch_v_cols) is faster, decline: both arrays
+  // in L2 with room to spare, so that its extra loads are cheap and the slab
+  // pipeline's start-up is not (vx and vy, us, slabs against columns: 48 x 48
+  // x 24 x 47 FP32 18.8 / 15.8 and FP64 19.9 / 17.9, 32^4 FP64 14.9 / 12.8, 64 x
+  // 49 x 48 x 50 FP32 26.0 / 21.9; 45 MB: 33.0 / 31.0, 64^4 FP32 41.5 / 45.4), or
+  // blocks that fill little of an SM's 512 threads (nvx = 72: 288; 80 x 90 x
+  // 72 x 70 FP32 120 / 82, FP64 179 / 157; nvx = 96, 384 threads: 74 / 84).
+  if (!c->fused_only && !bias && !c->slab &&
+      ((size_t)c->g.cells() * c->elem < (size_t)(40 << 20) || 512 / cfg.threads * cfg.threads < 320))
+    return VLP4D_ERR_UNSUPPORTED;
   PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (!encode) return VLP4D_ERR_UNSUPPORTED;
   const long long nxy = c->g.nxy();
@@ -526,7 +534,8 @@ int launch_advect_vxvy_tables(vlp4d_ctx *c, const void *fn, void *fnp1, const St
   a.nin = nin;
   a.C = cfg.C;
   a.Q = cfg.Q;
-  a.nseg = nvy / cfg.Q;
+  a.rows = nvy;
+  a.nseg = (nvy + cfg.Q - 1) / cfg.Q;
   a.nitems = (long long)nchunks * a.nseg;
   a.stages = cfg.stages;
   if (do_vx) a.tvx = *tvx;

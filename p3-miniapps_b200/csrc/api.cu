@@ -667,7 +667,20 @@ int vlp4d_steps(vlp4d_ctx *ctx, void *f_state, void *f_next, int iter0, int nste
     if (k + 1 == nsteps) break;
     // timestep.hpp:50-58 of step k, then :17-28 of step k+1, in one pass
     // where that pass is the faster choice.
-    rc = xyxy_join(ctx) ? launch_advect_xyxy(ctx, cur, oth, tx, ty, s) : VLP4D_ERR_UNSUPPORTED;
+    rc = VLP4D_ERR_UNSUPPORTED;
+    if (xyxy_join(ctx)) {
+      // By columns (FP32) where the plane kernel does not run: 99 x 101 x 77 x
+      // 83, five steps 3.35 ms against 3.91 with two passes, 45 x 39 x 51 x 43
+      // 0.50 against 0.56; where it runs it is faster, even in chunks of two
+      // rows (64 x 74 x 48 x 50: 0.755 against 0.828 ms).
+      if (ctx->dtype == VLP4D_F32 && !ctx->fused_only && !xyxy_runs(ctx)) {
+        StencilTable *x11 = nullptr, *y11 = nullptr;
+        if ((rc = ensure_xy11_table(ctx, 0, 0.5 * dt, &x11, s))) return rc;
+        if ((rc = ensure_xy11_table(ctx, 1, 0.5 * dt, &y11, s))) return rc;
+        rc = launch_xy_cols(ctx, cur, oth, x11, y11, 11, true, s);
+      }
+      if (rc == VLP4D_ERR_UNSUPPORTED) rc = launch_advect_xyxy(ctx, cur, oth, tx, ty, s);
+    }
     if (rc == VLP4D_ERR_UNSUPPORTED && !xyxy_join(ctx)) {
       if ((rc = advect_xy_impl(ctx, cur, oth, 0.5 * dt, false, s))) return rc;
       std::swap(cur, oth);

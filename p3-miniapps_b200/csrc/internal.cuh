@@ -248,6 +248,8 @@ int launch_advect_vxvy_tables(vlp4d_ctx *c, const void *fn, void *fnp1, const St
                               double bias_scale = 0.0);
 int launch_advect_xyxy(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTable *tx, const StencilTable *ty,
                        cudaStream_t s);
+// Whether the shape fits the joined plane pass.
+bool xyxy_runs(const vlp4d_ctx *c);
 // Whether the FP64 form of the joined pass (k_plane_xyxy64, row widths a
 // warp holds whole) runs for this context.
 bool xyxy64_available(const vlp4d_ctx *c);

@@ -67,3 +67,26 @@ def test_time_loop_matches_separate_steps(pkg, cuda, monkeypatch, n):
             p, q = q, p
         ctx.check()
         assert float((b - p).abs().max()) <= 3 * 2e-6 * float(f.max())
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("n", [(64, 8, 16, 43), (32, 32, 8, 131), (16, 16, 32, 7), (64, 64, 64, 61)])
+def test_uneven_vy_segments(pkg, cuda, monkeypatch, n, dtype):
+    """The v-slab pass where its vy segments do not divide nvy (the last one is
+    shorter), forced, against one thread per output; tolerances as for the
+    other fused-against-generic comparisons."""
+    torch = cuda
+    tol = 1e-14 if dtype == "f64" else 2e-7
+    with _ctx(pkg, monkeypatch, n, dtype, "fused") as fz, _ctx(pkg, monkeypatch, n, dtype, "generic") as gen:
+        f = fz.empty_f()
+        fz.init_case(f)
+        for which in (fz, gen):
+            h = torch.Generator().manual_seed(3)
+            which.ex.copy_(torch.randn(n[1], n[0], generator=h, dtype=torch.float64) * 3)
+            which.ey.copy_(torch.randn(n[1], n[0], generator=h, dtype=torch.float64) * 3)
+        for name in ("advect_vx", "advect_vy", "advect_vxvy"):
+            out, want = fz.empty_f(), gen.empty_f()
+            getattr(fz, name)(f, out, 0.2)
+            getattr(gen, name)(f, want, 0.2)
+            fz.check()
+            assert float((out - want).abs().max()) <= tol * float(want.abs().max()), name
