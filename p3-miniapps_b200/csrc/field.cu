@@ -32,10 +32,17 @@ __global__ void k_rho_partial(const T *__restrict__ f, double *__restrict__ part
   part[(long long)g * nxy + ixy] = s;
 }
 
-__global__ void __launch_bounds__(kMomentCells * kMomentSlices)
+template <int CELLS>
+__global__ void __launch_bounds__(kMomentThreads)
     k_rho_finish(const double *__restrict__ part, double *__restrict__ rho, long long nxy, int groups, double dvx,
                  double dvy) {
-  moment_finish(part, rho, nxy, groups, dvx, dvy);
+  moment_finish<CELLS, kMomentThreads / CELLS>(part, rho, nxy, groups, dvx, dvy);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kRhoSmallCells * kRhoSmallSlices)
+    k_rho_small(const T *__restrict__ f, double *__restrict__ rho, long long nxy, int nv, double dvx, double dvy) {
+  moment_small(f, rho, nxy, nv, dvx, dvy);
 }
 
 // ---- field_poisson pieces.
@@ -255,6 +262,17 @@ __global__ void k_transpose(const E *__restrict__ in, E *__restrict__ out, int r
 
 int launch_field_rho(vlp4d_ctx *c, const void *fn, cudaStream_t s) {
   const long long nxy = c->g.nxy(), nv = c->g.nv();
+  if (rho_small(nxy, nv)) {
+    const unsigned blocks = (unsigned)((nxy + kRhoSmallCells - 1) / kRhoSmallCells);
+    if (c->dtype == VLP4D_F64)
+      k_rho_small<double><<<blocks, kRhoSmallCells * kRhoSmallSlices, 0, s>>>((const double *)fn, c->rho, nxy, (int)nv,
+                                                                             c->g.dx[2], c->g.dx[3]);
+    else
+      k_rho_small<float><<<blocks, kRhoSmallCells * kRhoSmallSlices, 0, s>>>((const float *)fn, c->rho, nxy, (int)nv,
+                                                                            c->g.dx[2], c->g.dx[3]);
+    VLP4D_LAUNCH_CHECK();
+    return VLP4D_OK;
+  }
   const int threads = 256;
   const int groups = c->rho_groups;
   dim3 grid((unsigned)((nxy + threads - 1) / threads), (unsigned)groups);
@@ -268,8 +286,12 @@ int launch_field_rho(vlp4d_ctx *c, const void *fn, cudaStream_t s) {
 
 int launch_rho_finish(vlp4d_ctx *c, int groups, cudaStream_t s) {
   const long long nxy = c->g.nxy();
-  k_rho_finish<<<(unsigned)((nxy + kMomentCells - 1) / kMomentCells), kMomentCells * kMomentSlices, 0, s>>>(
-      c->rho_part, c->rho, nxy, groups, c->g.dx[2], c->g.dx[3]);
+  if (moment_wide(groups))
+    k_rho_finish<16><<<(unsigned)((nxy + 15) / 16), kMomentThreads, 0, s>>>(c->rho_part, c->rho, nxy, groups,
+                                                                            c->g.dx[2], c->g.dx[3]);
+  else
+    k_rho_finish<32><<<(unsigned)((nxy + 31) / 32), kMomentThreads, 0, s>>>(c->rho_part, c->rho, nxy, groups,
+                                                                            c->g.dx[2], c->g.dx[3]);
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }

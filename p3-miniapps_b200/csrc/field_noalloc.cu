@@ -86,10 +86,18 @@ __global__ void k_noalloc_rho_partial(const T *__restrict__ f, double *__restric
 }
 
 // The same fixed-order second stage as the context's (moment.cuh).
-__global__ void __launch_bounds__(kMomentCells * kMomentSlices)
+template <int CELLS>
+__global__ void __launch_bounds__(kMomentThreads)
     k_noalloc_rho_finish(const double *__restrict__ part, double *__restrict__ rho, long long nxy, int groups,
                          double dvx, double dvy) {
-  moment_finish(part, rho, nxy, groups, dvx, dvy);
+  moment_finish<CELLS, kMomentThreads / CELLS>(part, rho, nxy, groups, dvx, dvy);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kRhoSmallCells * kRhoSmallSlices)
+    k_noalloc_rho_small(const T *__restrict__ f, double *__restrict__ rho, long long nxy, int nv, double dvx,
+                        double dvy) {
+  moment_small(f, rho, nxy, nv, dvx, dvy);
 }
 
 }  // namespace
@@ -127,6 +135,17 @@ extern "C" int vlp4d_field_rho_noalloc(const void *fn, int dtype, int nx, int ny
   int sms = 0;
   int rc = noalloc_setup(dev, &part, &sms);
   if (rc) return rc;
+  // Few planes: one launch, as with a context.
+  if (rho_small(nxy, nv)) {
+    const unsigned blocks = (unsigned)((nxy + kRhoSmallCells - 1) / kRhoSmallCells);
+    const int nt = kRhoSmallCells * kRhoSmallSlices;
+    if (dtype == VLP4D_F64)
+      k_noalloc_rho_small<double><<<blocks, nt, 0, (cudaStream_t)stream>>>((const double *)fn, rho, nxy, (int)nv, dvx, dvy);
+    else
+      k_noalloc_rho_small<float><<<blocks, nt, 0, (cudaStream_t)stream>>>((const float *)fn, rho, nxy, (int)nv, dvx, dvy);
+    VLP4D_LAUNCH_CHECK();
+    return VLP4D_OK;
+  }
   // Same group count as a context would choose, limited by the scratch.
   long long groups = ((long long)sms * 8 * 256 + nxy - 1) / nxy;
   if (groups > nv) groups = nv;
@@ -141,8 +160,10 @@ extern "C" int vlp4d_field_rho_noalloc(const void *fn, int dtype, int nx, int ny
   else
     k_noalloc_rho_partial<float><<<grid, threads, 0, s>>>((const float *)fn, part, nxy, nv, (int)groups);
   VLP4D_LAUNCH_CHECK();
-  k_noalloc_rho_finish<<<(unsigned)((nxy + kMomentCells - 1) / kMomentCells), kMomentCells * kMomentSlices, 0, s>>>(
-      part, rho, nxy, (int)groups, dvx, dvy);
+  if (moment_wide((int)groups))
+    k_noalloc_rho_finish<16><<<(unsigned)((nxy + 15) / 16), kMomentThreads, 0, s>>>(part, rho, nxy, (int)groups, dvx, dvy);
+  else
+    k_noalloc_rho_finish<32><<<(unsigned)((nxy + 31) / 32), kMomentThreads, 0, s>>>(part, rho, nxy, (int)groups, dvx, dvy);
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }

@@ -3,9 +3,9 @@
 // FP64 partial sums part[group][ixy]).
 //
 // The groups are added in a fixed order that does not depend on the launch
-// shape: kMomentSlices contiguous ranges of groups, [s*G/S, (s+1)*G/S), each
-// summed in increasing group order, then the slices in increasing order.
-// Blocks of 32 cells x kMomentSlices slices sum the slices of a cell in
+// shape: S contiguous ranges of groups, [s*G/S, (s+1)*G/S), each summed in
+// increasing group order, then the slices in increasing order.  Blocks of
+// some cells x S slices sum the slices of a cell in
 // parallel (the partials of small grids are few cells of many groups; one
 // thread per cell left most of the GPU idle and the kernel bound by the
 // latency of its sequential loads).
@@ -13,9 +13,13 @@
 
 namespace vlp4d {
 
-constexpr int kMomentSlices = 16;
-constexpr int kMomentCells = 32;  // cells per block; blockDim = kMomentCells x kMomentSlices
+// Cells of a block and slices of the groups: 32 x 16, or 16 x 32 for many
+// groups (small planes: 1024 groups of 32 x 32 cells 3.9 us against 5.3; 74
+// groups of 128 x 128 cells 9.2 against 5.8).
+constexpr int kMomentThreads = 512;
+inline bool moment_wide(int groups) { return groups >= 512; }
 
+template <int kMomentCells, int kMomentSlices>
 __device__ __forceinline__ void moment_finish(const double *__restrict__ part, double *__restrict__ rho,
                                               long long nxy, int groups, double dvx, double dvy) {
   __shared__ double sl[kMomentSlices][kMomentCells];
@@ -43,6 +47,38 @@ __device__ __forceinline__ void moment_finish(const double *__restrict__ part, d
 #pragma unroll
     for (int k = 0; k < kMomentSlices; ++k) sum += sl[k][cx];
     rho[ixy] = sum * dvx * dvy;  // field.cpp:23 (sum * dvx * dvy)
+  }
+}
+
+// The whole moment in one launch where a cell has few planes: a block sums
+// kRhoSmallCells neighbouring cells in kRhoSmallSlices contiguous ranges of
+// the nv planes, then the ranges in order.  (16^4 FP64: 3.2 us against
+// 1.9 + 2.3 and a launch; moment, field and diagnostic 24.3 -> 21.4 us.)  Beyond
+// kRhoSmallPlanes planes, or where the cells alone fill the GPU, the two-stage
+// sum has the more loads in flight.
+constexpr int kRhoSmallCells = 16, kRhoSmallSlices = 32, kRhoSmallPlanes = 1024;
+inline bool rho_small(long long nxy, long long nv) { return nv <= kRhoSmallPlanes && nxy <= 8192; }
+
+template <typename T>
+__device__ __forceinline__ void moment_small(const T *__restrict__ f, double *__restrict__ rho, long long nxy, int nv,
+                                             double dvx, double dvy) {
+  __shared__ double sl[kRhoSmallSlices][kRhoSmallCells];
+  const int cx = threadIdx.x % kRhoSmallCells, s = threadIdx.x / kRhoSmallCells;
+  const long long ixy = (long long)blockIdx.x * kRhoSmallCells + cx;
+  const int v0 = nv * s / kRhoSmallSlices, v1 = nv * (s + 1) / kRhoSmallSlices;
+  double acc = 0.0;
+  if (ixy < nxy) {
+    const T *p = f + ixy + v0 * nxy;
+#pragma unroll 16
+    for (int v = v0; v < v1; ++v, p += nxy) acc += (double)__ldg(p);
+  }
+  sl[s][cx] = acc;
+  __syncthreads();
+  if (s == 0 && ixy < nxy) {
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < kRhoSmallSlices; ++k) sum += sl[k][cx];
+    rho[ixy] = sum * dvx * dvy;
   }
 }
 
