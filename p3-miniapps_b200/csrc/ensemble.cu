@@ -37,8 +37,7 @@
 // a tile of the new stage fences before reading.
 //
 // The field solve of a member (nx, ny <= 64) is a 2D DFT in FP64 shared
-// memory (direct sums with tabulated twiddles: a few hundred thousand
-// multiply-adds), the spectral solve of efield.cpp:43-105 (kx0 = 2*pi/xmax,
+// memory (two-factor sums with tabulated twiddles), the spectral solve of efield.cpp:43-105 (kx0 = 2*pi/xmax,
 // mode 0 zeroed), and the inverse DFT keeping the real part.
 #include <cmath>
 #include <cstdio>
@@ -46,6 +45,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "poisson.cuh"
 #include "stencil.cuh"
 #include "tma.cuh"
 
@@ -148,6 +148,7 @@ __device__ void ens_moment0(const EnsArgs &a, const EnsRun &R, const float *fin,
   double *pp = a.part + R.p_off + (long long)ivy * nxy;
   for (int q = threadIdx.x; q < nxy; q += blockDim.x) {
     double s = 0.;
+#pragma unroll 8
     for (int p = 0; p < nvx; ++p) s += (double)__ldcg(fin + row0 + (long long)p * nxy + q);
     pp[q] = s;
   }
@@ -667,30 +668,80 @@ __device__ void ens_vxvy(const EnsArgs &a, const EnsRun &R, const float *fin, fl
   }
 }
 
-// One 1D DFT pass over a (rows x len) complex array in shared memory:
-// out[r][k] = sum_j in[r][j] * w^(sign k j), w = exp(2 pi i / len); strides
-// select rows/columns.  tw[m] = (cos(2 pi m/len), sin(2 pi m/len)).
-__device__ void ens_dft(const double2 *in, double2 *out, int rows, int len, int rstride, int estride,
-                        const double2 *tw, double sign) {
+// 1D DFTs of the `rows` lines of length len of a complex array in shared
+// memory: out[r][k] = sum_j in[r][j] w^(sign k j), w = exp(2 pi i / len);
+// strides select rows or columns; tw[m] = (cos(2 pi m / len), sin(2 pi m /
+// len)).  By two factors, len = n1 n2, j = j1 n2 + j2, k = k1 + n1 k2: n1 + n2
+// terms per value instead of len (n1 = 1: a direct sum).  `buf` holds the
+// input; returns whichever of buf, tmp holds the result.  LINES_FIRST:
+// consecutive threads take consecutive lines (the columns of the array,
+// neighbours in memory), else consecutive values of a line.  Ends with a
+// barrier.
+template <bool LINES_FIRST>
+__device__ double2 *ens_dft(double2 *buf, double2 *tmp, int rows, int len, int rstride, int estride, const double2 *tw,
+                            double sign) {
+  const int n1 = dft_factor(len), n2 = len / n1;
+  const float inv_rows = 1.f / (float)rows, inv_len = 1.f / (float)len, inv_n1 = 1.f / (float)n1,
+              inv_n2 = 1.f / (float)n2;
+  const double2 *x = buf;
+  double2 *y = tmp;
+  if (n1 > 1) {
+    for (int o = threadIdx.x; o < rows * len; o += blockDim.x) {
+      const int a = LINES_FIRST ? div_small(o, rows, inv_rows) : div_small(o, len, inv_len);
+      const int q = LINES_FIRST ? a : o - a * len, r = LINES_FIRST ? o - a * rows : a;
+      const int k1 = div_small(q, n2, inv_n2), j2 = q - k1 * n2;
+      const double2 *p = buf + r * rstride + j2 * estride;
+      const int step = k1 * n2;
+      double sr = 0., si = 0.;
+      int m = 0;
+      for (int j = 0; j < n1; ++j) {
+        const double2 v = p[j * n2 * estride], w = tw[m];
+        const double wi = sign * w.y;
+        sr = fma(v.x, w.x, fma(-v.y, wi, sr));
+        si = fma(v.x, wi, fma(v.y, w.x, si));
+        m += step;
+        if (m >= len) m -= len;
+      }
+      const double2 w = tw[j2 * k1];
+      const double wi = sign * w.y;
+      tmp[r * rstride + q * estride] = make_double2(fma(sr, w.x, -si * wi), fma(sr, wi, si * w.x));
+    }
+    __syncthreads();
+    x = tmp;
+    y = buf;
+  }
   for (int o = threadIdx.x; o < rows * len; o += blockDim.x) {
-    const int r = o / len, k = o % len;
+    const int a = LINES_FIRST ? div_small(o, rows, inv_rows) : div_small(o, len, inv_len);
+    const int k = LINES_FIRST ? a : o - a * len, r = LINES_FIRST ? o - a * rows : a;
+    const int k2 = div_small(k, n1, inv_n1), k1 = k - k2 * n1;
+    const double2 *p = x + r * rstride + k1 * n2 * estride;
+    const int step = k2 * n1;
     double sr = 0., si = 0.;
     int m = 0;
-    for (int j = 0; j < len; ++j) {
-      const double2 v = in[r * rstride + j * estride];
-      const double2 w = tw[m];
+    for (int j = 0; j < n2; ++j) {
+      const double2 v = p[j * estride], w = tw[m];
       const double wi = sign * w.y;
       sr = fma(v.x, w.x, fma(-v.y, wi, sr));
       si = fma(v.x, wi, fma(v.y, w.x, si));
-      m += k;
+      m += step;
       if (m >= len) m -= len;
     }
-    out[r * rstride + k * estride] = make_double2(sr, si);
+    y[r * rstride + k * estride] = make_double2(sr, si);
   }
+  __syncthreads();
+  return y;
 }
 
 // Field solve of member R from its moment partials, diagnostic slot `iter`.
-// Shared memory: two complex (maxnxy) arrays and the twiddles.
+// Shared memory: two complex (maxnxy) arrays and the twiddles.  One CTA works
+// on it while the member's next stage waits, so its time is on the member's
+// chain of steps: Ex and Ey come out of one complex inverse transform of
+// ex_hat + i ey_hat (both Hermitian once the Nyquist column of ex_hat and the
+// Nyquist row of ey_hat are dropped, which is what keeping the real part of
+// either inverse alone does), the modes are formed once, and the transforms
+// take n1 + n2 terms per value.  60 members of 16 to 48 points a side, 20
+// steps: the kernel 10.5 -> 6.9 ms (before: direct sums, a division per term
+// of either inverse, the rows' partials loaded one after another).
 __device__ void ens_field(const EnsArgs &a, const EnsRun &R, int iter, unsigned char *smem) {
   const int nx = R.n[0], ny = R.n[1], nvy = R.n[3];
   const int nxy = nx * ny;
@@ -708,68 +759,54 @@ __device__ void ens_field(const EnsArgs &a, const EnsRun &R, int iter, unsigned 
     sincospi(2.0 * m / ny, &sn, &cs);
     twy[m] = make_double2(cs, sn);
   }
-  // rho = dvx dvy * (sum of the vy rows' partials, fixed order), as complex.
+  // rho = dvx dvy * (sum of the vy rows' partials, fixed order), as complex;
+  // sixteen rows' loads ahead of their additions.
   const double dvv = R.dx[2] * R.dx[3];
   const double *p = a.part + R.p_off;
   for (int c = threadIdx.x; c < nxy; c += blockDim.x) {
     double sum = 0.;
-    for (int v = 0; v < nvy; ++v) sum += __ldcg(p + (long long)v * nxy + c);
+    int v = 0;
+    for (; v + 16 <= nvy; v += 16) {
+      double t[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) t[k] = __ldcg(p + (long long)(v + k) * nxy + c);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) sum += t[k];
+    }
+    for (; v < nvy; ++v) sum += __ldcg(p + (long long)v * nxy + c);
     H1[c] = make_double2(sum * dvv, 0.);
   }
   __syncthreads();
-  ens_dft(H1, H2, ny, nx, nx, 1, twx, -1.);  // along x, every row
-  __syncthreads();
-  ens_dft(H2, H1, nx, ny, 1, nx, twy, -1.);  // along y, every column: H1 = rho_hat
-  __syncthreads();
+  double2 *z = ens_dft<false>(H1, H2, ny, nx, nx, 1, twx, -1.);                   // along x, every row
+  z = ens_dft<true>(z, z == H1 ? H2 : H1, nx, ny, 1, nx, twy, -1.);               // along y: rho_hat
   const double kx0 = 2 * M_PI / R.maxp[0], ky0 = 2 * M_PI / R.maxp[1];
   const double norm = 1.0 / ((double)nx * ny);
-  for (int comp = 0; comp < 2; ++comp) {
-    // H2 = inverse DFT along y of (-i k_comp / |k|^2 / (nx ny)) * rho_hat
-    // (mode 0 zeroed), column by column.
-    for (int o = threadIdx.x; o < nxy; o += blockDim.x) {
-      const int ix = o % nx, y = o / nx;
-      const double kx = (ix <= nx / 2 ? ix : ix - nx) * kx0;
-      double sr = 0., si = 0.;
-      int m = 0;
-      for (int iy = 0; iy < ny; ++iy) {
-        const double ky = (iy <= ny / 2 ? iy : iy - ny) * ky0;
-        const double k2 = kx * kx + ky * ky;
-        const double q = (ix == 0 && iy == 0) ? 0. : (comp == 0 ? kx : ky) / k2 * norm;
-        const double2 h = H1[iy * nx + ix];
-        const double vr = q * h.y, vi = -q * h.x;
-        const double2 w = twy[m];
-        sr = fma(vr, w.x, fma(-vi, w.y, sr));
-        si = fma(vr, w.y, fma(vi, w.x, si));
-        m += y;
-        if (m >= ny) m -= ny;
-      }
-      H2[o] = make_double2(sr, si);
-    }
-    __syncthreads();
-    // Real part of the inverse DFT along x, to the field arena.
-    double *e = a.fld + R.e_off + (long long)comp * nxy;
-    for (int o = threadIdx.x; o < nxy; o += blockDim.x) {
-      const int x = o % nx, y = o / nx;
-      double sr = 0.;
-      int m = 0;
-      for (int ix = 0; ix < nx; ++ix) {
-        const double2 v = H2[y * nx + ix];
-        const double2 w = twx[m];
-        sr = fma(v.x, w.x, fma(-v.y, w.y, sr));
-        m += x;
-        if (m >= nx) m -= nx;
-      }
-      e[o] = sr;
-    }
-    __syncthreads();
+  const float inv_nx = 1.f / (float)nx;
+  for (int o = threadIdx.x; o < nxy; o += blockDim.x) {
+    const int iy = div_small(o, nx, inv_nx), ix = o - iy * nx;
+    const double kx = (ix <= nx / 2 ? ix : ix - nx) * kx0, ky = (iy <= ny / 2 ? iy : iy - ny) * ky0;
+    const double k2 = kx * kx + ky * ky;
+    const double s = o == 0 ? 0. : norm / k2;
+    const double qx = 2 * ix == nx ? 0. : kx * s, qy = 2 * iy == ny ? 0. : ky * s;
+    // -i (qx + i qy) rho_hat
+    const double2 h = z[o];
+    z[o] = make_double2(fma(qx, h.y, qy * h.x), fma(qy, h.y, -qx * h.x));
+  }
+  __syncthreads();
+  z = ens_dft<true>(z, z == H1 ? H2 : H1, nx, ny, 1, nx, twy, 1.);
+  z = ens_dft<false>(z, z == H1 ? H2 : H1, ny, nx, nx, 1, twx, 1.);
+  double *ex = a.fld + R.e_off, *ey = ex + nxy;
+  for (int o = threadIdx.x; o < nxy; o += blockDim.x) {
+    ex[o] = z[o].x;
+    ey[o] = z[o].y;
   }
   // Energy: a fixed reduction order whatever the block size (lane l sums
   // cells l, l+32, ...; then a fixed shuffle tree), so the history does not
   // depend on the tile configuration.
   if (threadIdx.x < 32) {
-    const double *ex = a.fld + R.e_off, *ey = ex + nxy;
     double e2 = 0.;
-    for (int c = threadIdx.x; c < nxy; c += 32) e2 += ex[c] * ex[c] + ey[c] * ey[c];
+#pragma unroll 4
+    for (int c = threadIdx.x; c < nxy; c += 32) e2 += z[c].x * z[c].x + z[c].y * z[c].y;
     for (int o = 16; o > 0; o >>= 1) e2 += __shfl_down_sync(0xffffffffu, e2, o);
     if (threadIdx.x == 0) {
       const double en = sqrt(e2 * R.dx[0] * R.dx[1]);
@@ -898,24 +935,34 @@ __global__ void __launch_bounds__(512) k_ensemble(EnsArgs a) {
   }
 }
 
-__global__ void k_ens_init(EnsArgs a) {
+// f0 of every member: a block fills kInitPlanes (vx, vy) planes of its member
+// from one exponential per plane and one cosine per x and y (each cell's own
+// exponential and cosines cost 576 us over 49 M cells, 40 here).
+constexpr int kInitPlanes = 64;
+__global__ void __launch_bounds__(256) k_ens_init(EnsArgs a) {
   const EnsRun &R = a.runs[blockIdx.y];
-  const long long total = (long long)R.n[0] * R.n[1] * R.n[2] * R.n[3];
+  const int nx = R.n[0], ny = R.n[1], nvx = R.n[2];
+  const int nxy = nx * ny, planes = nvx * R.n[3];
+  const int p0 = blockIdx.x * kInitPlanes;
+  if (p0 >= planes) return;
+  const int np = planes - p0 < kInitPlanes ? planes - p0 : kInitPlanes;
+  __shared__ double cx[kEnsMaxN], cy[kEnsMaxN], m[kInitPlanes];
   const double PI = 3.14159265358979323846;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int ix = (int)(idx % R.n[0]);
-    long long q = idx / R.n[0];
-    const int iy = (int)(q % R.n[1]);
-    q /= R.n[1];
-    const int ivx = (int)(q % R.n[2]);
-    const int ivy = (int)(q / R.n[2]);
-    const double x = R.minp[0] + ix * R.dx[0];
-    const double y = R.minp[1] + iy * R.dx[1];
+  for (int i = threadIdx.x; i < nx; i += blockDim.x) cx[i] = cos(R.k * (R.minp[0] + i * R.dx[0]));
+  for (int i = threadIdx.x; i < ny; i += blockDim.x) cy[i] = cos(R.k * (R.minp[1] + i * R.dx[1]));
+  for (int i = threadIdx.x; i < np; i += blockDim.x) {
+    const int ivx = (p0 + i) % nvx, ivy = (p0 + i) / nvx;
     const double vx = R.minp[2] + ivx * R.dx[2];
     const double vy = R.minp[3] + ivy * R.dx[3];
-    const double val = (1. + R.amp * cos(R.k * x) + R.amp * cos(R.k * y)) * (exp(-0.5 * (vx * vx + vy * vy)) / (2 * PI));
-    a.F0[R.f_off + idx] = (float)val;
+    m[i] = exp(-0.5 * (vx * vx + vy * vy)) / (2 * PI);
+  }
+  __syncthreads();
+  const float inv_nx = 1.f / (float)nx;
+  for (int c = threadIdx.x; c < nxy; c += blockDim.x) {
+    const int iy = div_small(c, nx, inv_nx), ix = c - iy * nx;
+    const double shape = 1. + R.amp * cx[ix] + R.amp * cy[iy];
+    float *f = a.F0 + R.f_off + (long long)p0 * nxy + c;
+    for (int i = 0; i < np; ++i) f[(long long)i * nxy] = (float)(shape * m[i]);
   }
 }
 
@@ -968,7 +1015,7 @@ struct vlp4d_ensemble {
   unsigned long long *word = nullptr;
   unsigned int *done = nullptr;
   int *remaining = nullptr, *err = nullptr;
-  long long total_cells = 0, max_cells = 0;
+  long long total_cells = 0, max_planes = 0;
   int maxnxy = 0;
   // Tile configuration (vlp4d_ensemble_set_tiles / _autotune).
   int threads = 256, cc = 32, ctas_per_sm = 0;  // 0: as many as fit
@@ -1014,7 +1061,7 @@ EnsArgs ens_args(vlp4d_ensemble *E, int nsteps) {
 // Initial condition, scheduler reset and the persistent launch.
 int ens_launch(vlp4d_ensemble *E, int nsteps, cudaStream_t s) {
   const EnsArgs a = ens_args(E, nsteps);
-  dim3 ig((unsigned)((E->max_cells + 255) / 256 < 4096 ? (E->max_cells + 255) / 256 : 4096), (unsigned)E->nruns);
+  const dim3 ig((unsigned)((E->max_planes + kInitPlanes - 1) / kInitPlanes), (unsigned)E->nruns);
   k_ens_init<<<ig, 256, 0, s>>>(a);
   VLP4D_LAUNCH_CHECK();
   k_ens_reset<<<(E->nruns + 255) / 256, 256, 0, s>>>(a);
@@ -1145,7 +1192,7 @@ int vlp4d_ensemble_create(const vlp4d_ens_member *members, int nruns, int nsteps
       R.rows = (int)((R.n[3] + tiles - 1) / tiles);  // balanced tiles
     }
     E->total_cells += cells;
-    if (cells > E->max_cells) E->max_cells = cells;
+    if ((long long)R.n[2] * R.n[3] > E->max_planes) E->max_planes = (long long)R.n[2] * R.n[3];
     if (nxy > E->maxnxy) E->maxnxy = (int)nxy;
     E->host_runs.push_back(R);
   }

@@ -69,15 +69,6 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// The largest divisor of n up to its square root: the first factor of the
-// two-step DFT of lengths that are no power of two.
-__host__ __device__ inline int dft_factor(int n) {
-  int f = 1;
-  for (int d = 2; d * d <= n; ++d)
-    if (n % d == 0) f = d;
-  return f;
-}
-
 // DFT of `lines` contiguous lines of length n (line l at buf + l * n):
 // out[k] = sum_j in[j] w^(jk), w = exp(sign 2 pi i / n), tw[m] = exp(2 pi i
 // m / n) (conjugated for sign < 0).  The result is in buf or tmp (returned);

@@ -36,4 +36,13 @@ __device__ __forceinline__ void poisson_mode(int ix1, int ix2, int nx2, double2 
   }
 }
 
+// The largest divisor of n up to its square root: the first factor of the
+// two-step DFT of lengths that are no power of two.
+__host__ __device__ inline int dft_factor(int n) {
+  int f = 1;
+  for (int d = 2; d * d <= n; ++d)
+    if (n % d == 0) f = d;
+  return f;
+}
+
 }  // namespace vlp4d
