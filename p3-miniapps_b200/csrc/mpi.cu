@@ -993,18 +993,27 @@ __global__ void __launch_bounds__(256) k_mpi_advect_4d(const double *__restrict_
 // points and marches along vy: the coefficients its feet can reach (two more
 // points on each side of x, y and vx, five vy slabs) stay in a ring of six
 // shared-memory slabs, the sixth arriving by cp.async while a step computes.
-// A thread owns four cells at consecutive y: a coefficient row is read from
-// shared memory once for the four of them, 112 loads per cell instead of 256.
+// A thread owns four (EXACT: two) cells at consecutive y: a coefficient row is
+// read from shared memory once for all of them, 112 (160) loads per cell
+// instead of 256.
 //
 // Geometry of the tiles; vy in nseg segments of Q.
 struct Tile4 {
-  int W, YG, V;          // x extent, groups of four y, vx extent
-  int PX, RY, RV, slab;  // W + 4, 4 YG + 4, V + 4, PX * RY * RV
+  int R, W, YG, V;       // cells of a thread, x extent, groups of R y, vx extent
+  int PX, RY, RV, slab;  // W + 4, R YG + 4, V + 4, PX * RY * RV
   unsigned magic;        // ceil(2^32 / PX): i / PX for i < 2^16
   int nxt, nyt, nvt, Q, nseg;
   int nitems;
 };
-constexpr int kTileThreads = 256;
+// Cells of a thread (consecutive in y) and threads of a block.  Measured, us,
+// four cells and 256 threads (255 registers) against two and 512 (128): fused
+// 128 x 128 x 64 x 64 4343 / 5052, 64^4 1271 / 1349, 48 x 44 x 40 x 36 331 / 338;
+// EXACT, with twice the FP64 instructions per load, 6530 / 5474, 1891 / 1471 and
+// 443 / 366.  (Three and 384 threads: 19.9 ms at 128^4 against 16.6 for four.)
+template <bool EXACT>
+struct TileShape {
+  static constexpr int cells = EXACT ? 2 : 4, threads = EXACT ? 512 : 256;
+};
 constexpr int kRing = 6;
 
 // Weight j of the cubic B-spline at fractional offset p, for a j known at
@@ -1032,7 +1041,7 @@ constexpr int kTileY = 5;  // c1[3], y, first row
 // in the foot, at 64 per clock and SM) and the shared-memory pipe (112 loads
 // of 8 bytes per cell at 128 bytes per clock and SM) take about the same
 // time.  The sign of the field decides whether a cell's vx (vy) taps start
-// at -2 or -1; where the four cells of a thread disagree, the warp reads one
+// at -2 or -1; where the cells of a thread disagree, the warp reads one
 // slab more in that dimension and each cell's weight is 0 on the slab that
 // is not its own (EXACT skips it), so the lines where a field component changes sign cost a quarter more
 // there and not a second pass.  Cells whose x or y taps start at different
@@ -1042,17 +1051,17 @@ constexpr int kTileY = 5;  // c1[3], y, first row
 // 55 to 58 ms for two cells per thread from L1, whose warps ran both branches
 // wherever the two cells' first taps differed (26 ms where they hardly ever
 // did); FP64 pipe 48%, shared-memory pipe 51%, fixed-latency waits first (two
-// warps per scheduler: 255 registers).  384 threads of 168 registers, with
-// spills: 22.3 ms; sums along x first: 17.4 ms.
+// warps per scheduler); sums along x first: 17.4 ms.
 template <bool EXACT, bool MOMENT, int PXC>
-__global__ void __launch_bounds__(kTileThreads, 1)
+__global__ void __launch_bounds__(TileShape<EXACT>::threads, 1)
     k_mpi_advect_4d_tile(const double *__restrict__ c, double *__restrict__ fn, const double *__restrict__ ex,
                          const double *__restrict__ ey, HGrid h, Tile4 T, double dt, double *__restrict__ part,
                          double *__restrict__ l2, int *__restrict__ err) {
+  constexpr int kCells = TileShape<EXACT>::cells, kTileThreads = TileShape<EXACT>::threads;
   extern __shared__ __align__(16) double sm[];
   const int PX = PXC ? PXC : T.PX;
   const int RY = T.RY, slab = T.slab;
-  const int rows = 4 * T.YG, lines = T.W * T.V;
+  const int rows = kCells * T.YG, lines = T.W * T.V;
   double *fex = sm + kRing * slab, *fey = fex + PX * RY;
   double *xt = fey + PX * RY;         // [kTileX][lines]
   double *yt = xt + kTileX * lines;   // [2][kTileY][rows], by the parity of vy
@@ -1072,7 +1081,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     r /= T.nyt;
     const int vx0 = (r % T.nvt) * T.V, seg = r / T.nvt, vt = r % T.nvt;
     const int vy0 = seg * T.Q, vy1 = vy0 + T.Q < nvy ? vy0 + T.Q : nvy;
-    const int x = x0 + tx, y0 = yt0 + 4 * yg, ivx = vx0 + vl;
+    const int x = x0 + tx, y0 = yt0 + kCells * yg, ivx = vx0 + vl;
     const bool live = vl < T.V && x < nx && y0 < ny && ivx < nvx;
     __syncthreads();  // the item before has been read
     // Slab vy of the tile into ring slot `slot`; points past the halo (next
@@ -1131,7 +1140,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
       }
     };
     y_table(vy0);
-    double racc[4] = {0., 0., 0., 0.};
+    double racc[kCells] = {};
     int s0 = 0;  // ring slot of slab vy - 2
     for (int vy = vy0; vy < vy1; ++vy) {
       cp_async_wait_all();
@@ -1141,29 +1150,29 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         y_table(vy + 1);
       }
       if (live) {
-        double g[4][4];
-        bool ok[4];
+        double g[kCells][4];
+        bool ok[kCells];
         // The feet (foot4d, with the field from shared memory: its 3 x 3
         // points share their rows among the four cells).
         {
           const double *xl = xt + vl * T.W + tx;
-          const double *yl = yt + (vy & 1) * kTileY * rows + 4 * yg;
+          const double *yl = yt + (vy & 1) * kTileY * rows + kCells * yg;
           const int lx = (int)xl[5 * lines], ly = (int)yl[4 * rows];
-          bool infield = lx >= 0 && lx + 2 < PX && ly >= 0 && ly + 6 <= RY;
+          bool infield = lx >= 0 && lx + 2 < PX && ly >= 0 && ly + kCells + 2 <= RY;
 #pragma unroll
-          for (int q = 1; q < 4; ++q) infield &= yl[4 * rows + q] == yl[4 * rows] + q;
+          for (int q = 1; q < kCells; ++q) infield &= yl[4 * rows + q] == yl[4 * rows] + q;
           if (infield) {
             const double c0 = xl[0], c1 = xl[lines], c2 = xl[2 * lines];
-            double e1[4] = {0., 0., 0., 0.}, e2[4] = {0., 0., 0., 0.};
+            double e1[kCells] = {}, e2[kCells] = {};
             const double *p1 = fex + ly * PX + lx, *p2 = fey + ly * PX + lx;
 #pragma unroll
-            for (int k = 0; k < 6; ++k) {
+            for (int k = 0; k < kCells + 2; ++k) {
               const double a0 = p1[k * PX], a1 = p1[k * PX + 1], a2 = p1[k * PX + 2];
               const double b0 = p2[k * PX], b1 = p2[k * PX + 1], b2 = p2[k * PX + 2];
               const double ra = EXACT ? 0. : c0 * a0 + c1 * a1 + c2 * a2;
               const double rb = EXACT ? 0. : c0 * b0 + c1 * b1 + c2 * b2;
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
+              for (int q = 0; q < kCells; ++q) {
                 const int k1 = k - q;
                 if (k1 < 0 || k1 > 2) continue;
                 const double w = yl[k1 * rows + q];
@@ -1180,7 +1189,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
             const double xc = xl[3 * lines], vxc = xl[4 * lines];
             const double vyc = EXACT ? add(h.minp[3], mul((double)vy, h.dx[3])) : h.minp[3] + vy * h.dx[3];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < kCells; ++q) {
               const double yc = yl[3 * rows + q];
               double xs[4];
               if (EXACT) {
@@ -1203,7 +1212,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
             }
           } else {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < kCells; ++q) {
               const int iy = y0 + q < ny ? y0 + q : ny - 1;
               ok[q] = foot4d<EXACT>(h, ex, ey, x, iy, ivx, vy, dt, g[q]);
             }
@@ -1215,11 +1224,11 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         bool fast = true;
         int b2 = 0, b3 = 0;
         unsigned mx = 0, my = 0, m2 = 0, m3 = 0;
-        const unsigned all = y0 + 3 < ny ? 15u : (1u << (ny - y0)) - 1u;
-        double out[4] = {0., 0., 0., 0.};
-        double e0[4][4], e1[4][4], e2[4][4], p3[4];
+        const unsigned all = y0 + kCells <= ny ? (1u << kCells) - 1u : (1u << (ny - y0)) - 1u;
+        double out[kCells] = {};
+        double e0[kCells][4], e1[kCells][4], e2[kCells][4], p3[kCells];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < kCells; ++q) {
           const double f0 = floor(g[q][0]), f1 = floor(g[q][1]), f2 = floor(g[q][2]), f3 = floor(g[q][3]);
           const int a0 = (int)f0 - x + 1, a1 = (int)f1 - (y0 + q) + 1, a2 = (int)f2 - ivx + 1, a3 = (int)f3 - vy + 1;
           fast &= (ok[q] && (unsigned)(a0 | a1 | a2 | a3) < 2u) || y0 + q >= ny;
@@ -1244,18 +1253,18 @@ __global__ void __launch_bounds__(kTileThreads, 1)
           if (five3 && b3) { b3 = 0; m3 = all; }
           // The sum over the slabs for the cells whose x and y taps start at
           // (bx, by); MIX: some lane's cells differ in their first slab.
-          auto sweep = [&](auto mixed, unsigned bx, unsigned by, int n3, bool five2, double val[4]) {
+          auto sweep = [&](auto mixed, unsigned bx, unsigned by, int n3, bool five2, double val[kCells]) {
             constexpr bool MIX = decltype(mixed)::value;
             // First tap: local x = tx + 2 - 1 + (0 or -1) and so on.
-            const double *base = sm + ((vl + b2) * RY + 4 * yg + (int)by) * PX + tx + (int)bx;
+            const double *base = sm + ((vl + b2) * RY + kCells * yg + (int)by) * PX + tx + (int)bx;
             int slot = s0 + b3;
             if (slot >= kRing) slot -= kRing;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) val[q] = 0.;
+            for (int q = 0; q < kCells; ++q) val[q] = 0.;
             // The cells' vx weights on the five slabs (MIX) or the four.
-            double w2[4][MIX ? 5 : 4];
+            double w2[kCells][MIX ? 5 : 4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < kCells; ++q) {
               const bool later = MIX && ((m2 >> q) & 1);
 #pragma unroll
               for (int k = 0; k < (MIX ? 5 : 4); ++k)
@@ -1265,10 +1274,10 @@ __global__ void __launch_bounds__(kTileThreads, 1)
             for (int k3 = 0; k3 < n3; ++k3) {
               const double *sl = base + slot * slab;
               if (++slot == kRing) slot = 0;
-              double u[4] = {0., 0., 0., 0.}, w3[4];
-              bool in3[4];
+              double u[kCells] = {}, w3[kCells];
+              bool in3[kCells];
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
+              for (int q = 0; q < kCells; ++q) {
                 const int j = MIX ? k3 - (int)((m3 >> q) & 1) : k3;
                 in3[q] = !MIX || (j >= 0 && j < 4);
                 w3[q] = bspline_j<EXACT>(p3[q], j);
@@ -1280,12 +1289,12 @@ __global__ void __launch_bounds__(kTileThreads, 1)
                 const double *row = sl + k2 * RY * PX;
                 // EXACT sums along x first, as the reference does; otherwise y
                 // first: sixteen independent chains of four.
-                double s2[4], t[4][4];
+                double s2[kCells], t[kCells][4];
 #pragma unroll
-                for (int k = 0; k < 7; ++k) {
+                for (int k = 0; k < kCells + 3; ++k) {
                   const double v0 = row[k * PX], v1 = row[k * PX + 1], v2 = row[k * PX + 2], v3 = row[k * PX + 3];
 #pragma unroll
-                  for (int q = 0; q < 4; ++q) {
+                  for (int q = 0; q < kCells; ++q) {
                     const int k1 = k - q;
                     if (k1 < 0 || k1 > 3) continue;
                     if (EXACT) {
@@ -1304,7 +1313,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
                   }
                 }
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
+                for (int q = 0; q < kCells; ++q) {
                   const bool later = MIX && ((m2 >> q) & 1);
                   const bool in2 = k2 == 0 ? !later : (k2 == 4 ? later : true);
                   if (EXACT) {
@@ -1317,7 +1326,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
               }
               if (!EXACT) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) val[q] = fma(u[q], w3[q], val[q]);
+                for (int q = 0; q < kCells; ++q) val[q] = fma(u[q], w3[q], val[q]);
               }
             }
           };
@@ -1329,15 +1338,15 @@ __global__ void __launch_bounds__(kTileThreads, 1)
             const unsigned bx = (mx >> q0) & 1, by = (my >> q0) & 1;
             const unsigned take = rem & (bx ? mx : ~mx) & (by ? my : ~my);
             rem &= ~take;
-            double val[4];
+            double val[kCells];
             if (five2 || five3) sweep(std::true_type{}, bx, by, five3 ? 5 : 4, five2, val);
             else sweep(std::false_type{}, bx, by, 4, false, val);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) out[q] = (take >> q) & 1 ? val[q] : out[q];
+            for (int q = 0; q < kCells; ++q) out[q] = (take >> q) & 1 ? val[q] : out[q];
           } while (__any_sync(act, rem != 0));
         } else {
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
+          for (int q = 0; q < kCells; ++q) {
             if (y0 + q < ny) {
               // The foot again: it is rarely needed and not kept.
               double gq[4];
@@ -1348,7 +1357,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         }
         double *o = fn + h.at(x, y0, ivx, vy);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < kCells; ++q) {
           if (y0 + q < ny) {
             o[q * h.s[1]] = out[q];
             if (MOMENT) {
@@ -1366,7 +1375,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
       const int cells = T.W * rows;
       if (vl < T.V) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) sm[vl * cells + (4 * yg + q) * T.W + tx] = live ? racc[q] : 0.;
+        for (int q = 0; q < kCells; ++q) sm[vl * cells + (kCells * yg + q) * T.W + tx] = live ? racc[q] : 0.;
       }
       __syncthreads();
       double *dst = part + (long long)(vt * T.nseg + seg) * nx * ny;
@@ -1722,7 +1731,7 @@ int launch_advect_4d(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn,
 // The ring, the field around the tile, the predictor's x and y parts.
 size_t tile4_smem(const Tile4 &T) {
   return sizeof(double) * ((size_t)kRing * T.slab + 2 * (size_t)T.PX * T.RY + (size_t)kTileX * T.W * T.V +
-                           2 * (size_t)kTileY * 4 * T.YG) +
+                           2 * (size_t)kTileY * T.R * T.YG) +
          sizeof(int) * (size_t)T.RY * T.RV;
 }
 
@@ -1732,26 +1741,27 @@ size_t tile4_smem(const Tile4 &T) {
 // the grid's edge idles, and every segment starts with five slabs and their
 // latency, about two steps' worth.  False: nothing fits (or more partials
 // than the context holds), and the cell-per-thread kernel runs (48 x 44 x 40
-// x 36 in the reference's arithmetic: 0.555 ms against 0.452 for the tiles).
-bool tile4_config(const vlp4d_ctx *c, const HGrid &h, bool moment, Tile4 &T) {
+// x 36 in the reference's arithmetic: 0.555 ms against 0.366 for the tiles).
+bool tile4_config(const vlp4d_ctx *c, const HGrid &h, int cells, int threads, bool moment, Tile4 &T) {
   const int lim = smem_limit(c) - 1024;
   const long long nx = h.n[0], ny = h.n[1], nvx = h.n[2], nvy = h.n[3];
   Tile4 t;
+  t.R = cells;
   t.nxt = (int)((nx + 31) / 32);
   t.W = (int)((nx + t.nxt - 1) / t.nxt);
   t.PX = t.W + 4;
   t.magic = (unsigned)(((1ULL << 32) + t.PX - 1) / t.PX);
   double best = 0.;
-  for (int yg = 1; yg <= 8; ++yg)
+  for (int yg = 1; yg <= 16; ++yg)
     for (int v = 1; v <= 16; ++v) {
-      if (t.W * yg * v > kTileThreads) continue;
+      if (t.W * yg * v > threads) continue;
       t.YG = yg;
       t.V = v;
-      t.RY = 4 * yg + 4;
+      t.RY = cells * yg + 4;
       t.RV = v + 4;
       t.slab = t.PX * t.RY * t.RV;
       if ((long long)tile4_smem(t) > lim) continue;
-      const long long nyt = (ny + 4 * yg - 1) / (4 * yg), nvt = (nvx + v - 1) / v;
+      const long long nyt = (ny + cells * yg - 1) / (cells * yg), nvt = (nvx + v - 1) / v;
       if (nyt * nvt * t.nxt > (1 << 24)) continue;
       for (long long nseg = 1; nseg <= nvy && nseg <= 64; ++nseg) {
         const long long Q = (nvy + nseg - 1) / nseg;
@@ -1782,7 +1792,7 @@ int run_advect_4d_tile(vlp4d_ctx *c, const HGrid &h, const Tile4 &T, const doubl
   const size_t smem = tile4_smem(T);
   VLP4D_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = T.nitems < c->num_sms ? T.nitems : c->num_sms;
-  k<<<grid, kTileThreads, smem, s>>>(c4, fn, c->ex, c->ey, h, T, dt, c->rho_part, c->mpi_part, c->d_err);
+  k<<<grid, TileShape<EXACT>::threads, smem, s>>>(c4, fn, c->ex, c->ey, h, T, dt, c->rho_part, c->mpi_part, c->d_err);
   VLP4D_LAUNCH_CHECK();
   if (blocks) *blocks = grid;
   return VLP4D_OK;
@@ -1795,7 +1805,8 @@ template <bool EXACT, bool MOMENT>
 int launch_advect_4d_any(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn, double dt, int *groups,
                          long long *blocks, cudaStream_t s) {
   Tile4 T;
-  if (!c->fused || !tile4_config(c, h, MOMENT, T)) return launch_advect_4d<EXACT, MOMENT>(c, h, c4, fn, dt, groups, blocks, s);
+  if (!c->fused || !tile4_config(c, h, TileShape<EXACT>::cells, TileShape<EXACT>::threads, MOMENT, T))
+    return launch_advect_4d<EXACT, MOMENT>(c, h, c4, fn, dt, groups, blocks, s);
   if (groups) *groups = T.nvt * T.nseg;
   if (T.PX == 36) return run_advect_4d_tile<EXACT, MOMENT, 36>(c, h, T, c4, fn, dt, blocks, s);
   return run_advect_4d_tile<EXACT, MOMENT, 0>(c, h, T, c4, fn, dt, blocks, s);
