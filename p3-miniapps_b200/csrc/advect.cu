@@ -29,6 +29,8 @@ struct VtableJob {
   int C;
 };
 __global__ void k_build_vtable(VtableJob j0, VtableJob j1, int lines, double dt) {
+  pdl_wait();
+  pdl_trigger();
   const int line = blockIdx.x * blockDim.x + threadIdx.x;
   const bool on = line < lines;
   const VtableJob j = blockIdx.y ? j1 : j0;
@@ -371,7 +373,8 @@ int build_v_tables(vlp4d_ctx *c, double dt, bool vx, bool vy, cudaStream_t s) {
                      c->tab_vy.span_C ? c->tab_vy.span : nullptr, c->tab_vy.span_C};
   }
   if (!njobs) return VLP4D_OK;
-  k_build_vtable<<<dim3((unsigned)blocks, (unsigned)njobs), threads, 0, s>>>(jobs[0], jobs[njobs - 1], lines, dt);
+  VLP4D_CUDA_TRY(launch_pdl(k_build_vtable, dim3((unsigned)blocks, (unsigned)njobs), dim3(threads), 0, s, jobs[0],
+                            jobs[njobs - 1], lines, dt));
   VLP4D_LAUNCH_CHECK();
   if (vx) c->tab_vx.valid = true;
   if (vy) c->tab_vy.valid = true;

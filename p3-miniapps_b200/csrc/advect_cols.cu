@@ -70,6 +70,7 @@ constexpr int kColsWidth = 128;   // most columns of a tile
 // branch per row and divisions in the loads: 461, 780 and 33 us.
 template <typename T, int TX, int TY, int RM, bool RHO>
 __global__ void __launch_bounds__(kColsThreads, 2) k_xy_cols(XyCols a) {
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char csm[];
   T *tile = reinterpret_cast<T *>(csm);
   constexpr int HX = TX ? TX - 1 : 0, HY = TY ? TY - 1 : 0;
@@ -201,6 +202,7 @@ constexpr int kVColsThreads = 128;
 // one thread per output; 127 x 127 x 96 x 96, 626 us (3.8 TB/s).
 template <typename T, bool DVX, bool DVY, int V>
 __global__ void __launch_bounds__(kVColsThreads, 4) k_v_cols(VCols a) {
+  pdl_wait();
   const unsigned gid = blockIdx.x * kVColsThreads + threadIdx.x;
   if (gid >= (unsigned)a.nxy * (unsigned)a.ngx) return;
   const int col = (int)(gid % (unsigned)a.nxy), ivx0 = (int)(gid / (unsigned)a.nxy) * V;
@@ -210,12 +212,12 @@ __global__ void __launch_bounds__(kVColsThreads, 4) k_v_cols(VCols a) {
   T wx[6], wy[6];
   int jx = ivx0, jy = iv0;
   if (DVX) {
-    load_weights(WeightsOf<T>::get(a.tvx), col, wx);
-    jx += a.tvx.m[col];
+    load_weights_cg(WeightsOf<T>::get(a.tvx), col, wx);
+    jx += __ldcg(a.tvx.m + col);
   }
   if (DVY) {
-    load_weights(WeightsOf<T>::get(a.tvy), col, wy);
-    jy = (iv0 + a.tvy.m[col]) % a.nvy;
+    load_weights_cg(WeightsOf<T>::get(a.tvy), col, wy);
+    jy = (iv0 + __ldcg(a.tvy.m + col)) % a.nvy;
   }
   int off[NT];
   jx %= a.nvx;
@@ -345,7 +347,8 @@ int run_v_cols(vlp4d_ctx *c, VCols &a, cudaStream_t s) {
       a.Q = Q;
     }
   }
-  k_v_cols<T, DVX, DVY, V><<<dim3((unsigned)blocks, (unsigned)((a.nvy + a.Q - 1) / a.Q)), kVColsThreads, 0, s>>>(a);
+  VLP4D_CUDA_TRY(launch_pdl(k_v_cols<T, DVX, DVY, V>, dim3((unsigned)blocks, (unsigned)((a.nvy + a.Q - 1) / a.Q)),
+                            dim3(kVColsThreads), 0, s, a));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }

@@ -200,6 +200,7 @@ __device__ __forceinline__ void sweep_y_pairs(const double *src, int nx, int h, 
 // for the whole kernel; blockDim = (nx/4) * (R/RT).
 template <typename T, int NX, int RT, bool DX, bool DY, bool RHO, bool INPLACE = false>
 __global__ void __launch_bounds__(512) k_plane(PlaneArgs a) {
+  pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem[];
   const int nx = NX ? NX : a.nx;
   const int ny = a.ny, R = a.R, S = a.stages;
@@ -646,6 +647,7 @@ __device__ __forceinline__ int xyxy_swz(int chunk) { return chunk ^ ((chunk >> 3
 // stencils has no use for one).
 template <typename T, int NX, int RT, bool X8 = false, bool RHO = true>
 __global__ void __launch_bounds__(512) k_plane_xyxy(PlaneArgs a) {
+  pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem[];
   const int nx = NX ? NX : a.nx;
   const int ny = a.ny, R = a.R, S = a.stages;
@@ -884,6 +886,7 @@ __device__ __forceinline__ void x11_pair_row(const double *row, int a0, int nx, 
 
 template <int NX, int RT, bool RHO = true>
 __global__ void __launch_bounds__(512) k_plane_xyxy64(PlaneArgs a) {
+  pdl_trigger();
   using T = double;
   extern __shared__ __align__(128) unsigned char smem[];
   const int nx = NX ? NX : a.nx;

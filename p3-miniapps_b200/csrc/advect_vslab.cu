@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(512) k_vslab(const __grid_constant__ CUtensorM
     }
     mbar_fence_init();
   }
+  pdl_wait();
   __syncthreads();
 
   // Look-ahead cursor: slab S of the sequence (the first S are issued here).
@@ -202,9 +203,9 @@ __global__ void __launch_bounds__(512) k_vslab(const __grid_constant__ CUtensorM
     {
       int j = vx0;
       if (DVX) {
-        j += __ldg(a.tvx.m + ixy);
+        j += __ldcg(a.tvx.m + ixy);
         if (j >= nvx) j -= nvx;
-        load_weights(WeightsOf<T>::get(a.tvx), ixy, wvx);
+        load_weights_cg(WeightsOf<T>::get(a.tvx), ixy, wvx);
       }
 #pragma unroll
       for (int q = 0; q < V + 5; ++q) {
@@ -213,11 +214,11 @@ __global__ void __launch_bounds__(512) k_vslab(const __grid_constant__ CUtensorM
       }
     }
     if (DVY) {
-      lag0 = 5 + signed_offset(__ldg(a.tvy.m + ixy), a.nvy) - a.span[cc].x;
-      load_weights(WeightsOf<T>::get(a.tvy), ixy, wvy);
+      lag0 = 5 + signed_offset(__ldcg(a.tvy.m + ixy), a.nvy) - a.span[cc].x;
+      load_weights_cg(WeightsOf<T>::get(a.tvy), ixy, wvy);
     }
     constexpr bool has_bias = BIAS;
-    const double bias = BIAS ? a.bias_scale * __ldg(a.bias + ixy) : 0.0;
+    const double bias = BIAS ? a.bias_scale * __ldcg(a.bias + ixy) : 0.0;
     // Output pointer of the next row this thread writes.
     T *orow = static_cast<T *>(a.fout) + ixy + vstride * vx0 + ystride * (long long)sg * a.Q;
     // Ring of vx-swept rows, slot = t % 6 (static after unrolling).  FP64:
@@ -456,7 +457,7 @@ int run_vslab(vlp4d_ctx *c, const CUtensorMap &map, const VslabArgs &args, const
   if (cap > 0 && per_sm > cap) per_sm = cap;
   long long grid = (long long)per_sm * c->num_sms;
   if (grid > args.nitems) grid = args.nitems;
-  kern<<<(unsigned)grid, cfg.threads, cfg.smem, s>>>(map, args);
+  VLP4D_CUDA_TRY(launch_pdl(kern, dim3((unsigned)grid), dim3(cfg.threads), cfg.smem, s, map, args));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }

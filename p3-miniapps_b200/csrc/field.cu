@@ -21,6 +21,7 @@ namespace {
 template <typename T>
 __global__ void k_rho_partial(const T *__restrict__ f, double *__restrict__ part, long long nxy, long long nv,
                               int groups) {
+  pdl_trigger();
   const long long ixy = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const int g = blockIdx.y;
   if (ixy >= nxy) return;
@@ -36,12 +37,15 @@ template <int CELLS>
 __global__ void __launch_bounds__(kMomentThreads)
     k_rho_finish(const double *__restrict__ part, double *__restrict__ rho, long long nxy, int groups, double dvx,
                  double dvy) {
+  pdl_wait();
+  pdl_trigger();
   moment_finish<CELLS, kMomentThreads / CELLS>(part, rho, nxy, groups, dvx, dvy);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kRhoSmallCells * kRhoSmallSlices)
     k_rho_small(const T *__restrict__ f, double *__restrict__ rho, long long nxy, int nv, double dvx, double dvy) {
+  pdl_trigger();
   moment_small(f, rho, nxy, nv, dvx, dvy);
 }
 
@@ -92,10 +96,9 @@ __device__ __forceinline__ void kahan_add(double &sum, double &c, double x) {
   sum = t;
 }
 
-__global__ void k_diags(const double *__restrict__ rho, const double *__restrict__ ex, const double *__restrict__ ey,
-                        long long n, double dx, double dy, double *__restrict__ nrj_hist,
-                        double *__restrict__ mass_hist, double *__restrict__ nrjx_hist,
-                        double *__restrict__ nrjy_hist, int iter) {
+__global__ void k_diags(const double *rho, const double *ex, const double *ey,
+                        long long n, double dx, double dy, double *nrj_hist, double *mass_hist, double *nrjx_hist, double *nrjy_hist, int iter) {
+  pdl_wait();
   // Kahan sums of rho, Ex^2 + Ey^2, Ex^2, Ey^2.
   // Each thread's elements in order; the loads of four of them are issued
   // before their adds so that their latencies overlap.
@@ -286,12 +289,10 @@ int launch_field_rho(vlp4d_ctx *c, const void *fn, cudaStream_t s) {
 
 int launch_rho_finish(vlp4d_ctx *c, int groups, cudaStream_t s) {
   const long long nxy = c->g.nxy();
-  if (moment_wide(groups))
-    k_rho_finish<16><<<(unsigned)((nxy + 15) / 16), kMomentThreads, 0, s>>>(c->rho_part, c->rho, nxy, groups,
-                                                                            c->g.dx[2], c->g.dx[3]);
-  else
-    k_rho_finish<32><<<(unsigned)((nxy + 31) / 32), kMomentThreads, 0, s>>>(c->rho_part, c->rho, nxy, groups,
-                                                                            c->g.dx[2], c->g.dx[3]);
+  const bool wide = moment_wide(groups);
+  const int cells = wide ? 16 : 32;
+  VLP4D_CUDA_TRY(launch_pdl(wide ? k_rho_finish<16> : k_rho_finish<32>, dim3((unsigned)((nxy + cells - 1) / cells)),
+                            dim3(kMomentThreads), 0, s, c->rho_part, c->rho, nxy, groups, c->g.dx[2], c->g.dx[3]));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }
@@ -334,8 +335,8 @@ int launch_field_poisson(vlp4d_ctx *c, cudaStream_t s) {
 }
 
 int launch_diags(vlp4d_ctx *c, int iter, cudaStream_t s) {
-  k_diags<<<1, 1024, 0, s>>>(c->rho, c->ex, c->ey, c->g.nxy(), c->g.dx[0], c->g.dx[1], c->nrj, c->mass, c->nrjx,
-                             c->nrjy, iter);
+  VLP4D_CUDA_TRY(launch_pdl(k_diags, dim3(1), dim3(1024), 0, s, c->rho, c->ex, c->ey, c->g.nxy(), c->g.dx[0], c->g.dx[1],
+                            c->nrj, c->mass, c->nrjx, c->nrjy, iter));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }
@@ -343,8 +344,10 @@ int launch_diags(vlp4d_ctx *c, int iter, cudaStream_t s) {
 int diags_async(vlp4d_ctx *c, int iter, cudaStream_t s) {
   VLP4D_CUDA_TRY(cudaEventRecord(c->ev_fork, s));
   VLP4D_CUDA_TRY(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-  int rc = launch_diags(c, iter, c->side);
-  if (rc) return rc;
+  // An ordinary launch: it follows an event, not a kernel.
+  k_diags<<<1, 1024, 0, c->side>>>(c->rho, c->ex, c->ey, c->g.nxy(), c->g.dx[0], c->g.dx[1], c->nrj, c->mass, c->nrjx,
+                                   c->nrjy, iter);
+  VLP4D_LAUNCH_CHECK();
   VLP4D_CUDA_TRY(cudaEventRecord(c->ev_join, c->side));
   return VLP4D_OK;
 }

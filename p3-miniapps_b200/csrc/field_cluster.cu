@@ -235,6 +235,8 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster(FieldArgs a) {
     sincospi(2.0 * m / ny, &sn, &cs);
     twy[m] = make_double2(cs, sn);
   }
+  pdl_wait();
+  pdl_trigger();
   // 1. Own rows along x (the last CTAs may have fewer than R, or none).
   const int iy0 = (int)c * R;
   const int nr = ny - iy0 < R ? (ny - iy0 > 0 ? ny - iy0 : 0) : R;
@@ -347,6 +349,8 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster_t(FieldTArgs a)
     sincospi(2.0 * m / ny, &sn, &cs);
     twy[m] = make_double2(cs, sn);
   }
+  pdl_wait();
+  pdl_trigger();
   const int iy0 = (int)c * R;
   const int nr = ny - iy0 < R ? (ny - iy0 > 0 ? ny - iy0 : 0) : R;
   for (int i = threadIdx.x; i < nr * nx; i += blockDim.x) {
@@ -415,8 +419,10 @@ cudaLaunchConfig_t field_config(int nx, int ny, int ctas, cudaLaunchAttribute *a
   attr->val.clusterDim.x = ctas;
   attr->val.clusterDim.y = 1;
   attr->val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cfg;
 }
 
@@ -429,8 +435,8 @@ bool cluster_fits(int nx, int ny) {
     cudaGetLastError();
     return false;
   }
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = field_config(nx, ny, C, &attr, 0);
+  cudaLaunchAttribute attr[2] = {};
+  const cudaLaunchConfig_t cfg = field_config(nx, ny, C, attr, 0);
   int clusters = 0;
   if (cudaOccupancyMaxActiveClusters(&clusters, k_field_cluster<C, POW2>, &cfg) != cudaSuccess || clusters < 1) {
     cudaGetLastError();
@@ -448,8 +454,8 @@ bool cluster_t_fits(int nx, int ny) {
     cudaGetLastError();
     return false;
   }
-  cudaLaunchAttribute attr;
-  cudaLaunchConfig_t cfg = field_config(nx, ny, C, &attr, 0);
+  cudaLaunchAttribute attr[2] = {};
+  cudaLaunchConfig_t cfg = field_config(nx, ny, C, attr, 0);
   cfg.dynamicSmemBytes = smem;
   int clusters = 0;
   if (cudaOccupancyMaxActiveClusters(&clusters, k_field_cluster_t<C, POW2>, &cfg) != cudaSuccess || clusters < 1) {
@@ -509,8 +515,8 @@ int launch_field_transpose_cluster(vlp4d_ctx *c, const double *gex, const double
   a.nx = nx;
   a.ny = ny;
   a.norm = 1.0 / ((double)nx * ny);
-  cudaLaunchAttribute attr;
-  cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, &attr, s);
+  cudaLaunchAttribute attr[2] = {};
+  cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, attr, s);
   cfg.dynamicSmemBytes = field_t_bytes(nx, ny, c->field_cluster);
   const bool p2 = pow2_plane(nx, ny);
   if (c->field_cluster == 16)
@@ -531,8 +537,8 @@ int launch_field_cluster(vlp4d_ctx *c, double offset, cudaStream_t s) {
   a.kx0 = 2 * M_PI / c->g.maxp[0];  // efield.cpp:44-45: 2*pi / maxPhy
   a.ky0 = 2 * M_PI / c->g.maxp[1];
   a.normcoeff = 1.0 / (double)(nx * ny);
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, &attr, s);
+  cudaLaunchAttribute attr[2] = {};
+  const cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, attr, s);
   const bool p2 = pow2_plane(nx, ny);
   if (c->field_cluster == 16)
     VLP4D_CUDA_TRY(cudaLaunchKernelEx(&cfg, p2 ? k_field_cluster<16, true> : k_field_cluster<16, false>, a));

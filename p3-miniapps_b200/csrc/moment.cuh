@@ -34,11 +34,11 @@ __device__ __forceinline__ void moment_finish(const double *__restrict__ part, d
     for (; g + 8 <= g1; g += 8) {
       double v[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = part[(long long)(g + k) * nxy + ixy];
+      for (int k = 0; k < 8; ++k) v[k] = __ldcg(part + (long long)(g + k) * nxy + ixy);
 #pragma unroll
       for (int k = 0; k < 8; ++k) acc += v[k];
     }
-    for (; g < g1; ++g) acc += part[(long long)g * nxy + ixy];
+    for (; g < g1; ++g) acc += __ldcg(part + (long long)g * nxy + ixy);
   }
   sl[s][cx] = acc;
   __syncthreads();

@@ -135,4 +135,12 @@ __device__ __forceinline__ void load_weights(const T *__restrict__ w, long long 
   for (int k = 0; k < 6; ++k) out[k] = __ldg(w + 6 * line + k);
 }
 
+// The same through L2, for tables that the kernel before may still be writing
+// when this one starts.
+template <typename T>
+__device__ __forceinline__ void load_weights_cg(const T *w, long long line, T (&out)[6]) {
+#pragma unroll
+  for (int k = 0; k < 6; ++k) out[k] = __ldcg(w + 6 * line + k);
+}
+
 }  // namespace vlp4d
