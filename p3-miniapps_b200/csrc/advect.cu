@@ -373,7 +373,7 @@ int build_v_tables(vlp4d_ctx *c, double dt, bool vx, bool vy, cudaStream_t s) {
                      c->tab_vy.span_C ? c->tab_vy.span : nullptr, c->tab_vy.span_C};
   }
   if (!njobs) return VLP4D_OK;
-  VLP4D_CUDA_TRY(launch_pdl(k_build_vtable, dim3((unsigned)blocks, (unsigned)njobs), dim3(threads), 0, s, jobs[0],
+  VLP4D_CUDA_TRY(launch_dep(c, k_build_vtable, dim3((unsigned)blocks, (unsigned)njobs), dim3(threads), 0, s, jobs[0],
                             jobs[njobs - 1], lines, dt));
   VLP4D_LAUNCH_CHECK();
   if (vx) c->tab_vx.valid = true;

@@ -70,6 +70,8 @@ constexpr int kColsWidth = 128;   // most columns of a tile
 // branch per row and divisions in the loads: 461, 780 and 33 us.
 template <typename T, int TX, int TY, int RM, bool RHO>
 __global__ void __launch_bounds__(kColsThreads, 2) k_xy_cols(XyCols a) {
+  pdl_wait();
+  pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(16) unsigned char csm[];
   T *tile = reinterpret_cast<T *>(csm);
@@ -203,6 +205,8 @@ constexpr int kVColsThreads = 128;
 template <typename T, bool DVX, bool DVY, int V>
 __global__ void __launch_bounds__(kVColsThreads, 4) k_v_cols(VCols a) {
   pdl_wait();
+  pdl_trigger();
+  pdl_trigger();
   const unsigned gid = blockIdx.x * kVColsThreads + threadIdx.x;
   if (gid >= (unsigned)a.nxy * (unsigned)a.ngx) return;
   const int col = (int)(gid % (unsigned)a.nxy), ivx0 = (int)(gid / (unsigned)a.nxy) * V;
@@ -233,7 +237,7 @@ __global__ void __launch_bounds__(kVColsThreads, 4) k_v_cols(VCols a) {
   auto load = [&](int j, T (&t)[NT]) {
     const T *row = fin + (long long)j * ystride;
 #pragma unroll
-    for (int k = 0; k < NT; ++k) t[k] = __ldg(row + off[k]);
+    for (int k = 0; k < NT; ++k) t[k] = row[off[k]];
   };
   load(jy, cur);
   for (int r0 = 0; r0 < rows; r0 += 6) {
@@ -287,7 +291,7 @@ int run_xy_cols(vlp4d_ctx *c, XyCols &a, cudaStream_t s) {
   G = (planes + per - 1) / per;
   if (G * tiles > 0x7fffffffLL) return VLP4D_ERR_UNSUPPORTED;
   a.G = (int)G;
-  k<<<(unsigned)(G * tiles), threads, smem, s>>>(a);
+  VLP4D_CUDA_TRY(launch_dep(c, k, dim3((unsigned)(G * tiles)), dim3(threads), smem, s, a));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }
@@ -347,7 +351,7 @@ int run_v_cols(vlp4d_ctx *c, VCols &a, cudaStream_t s) {
       a.Q = Q;
     }
   }
-  VLP4D_CUDA_TRY(launch_pdl(k_v_cols<T, DVX, DVY, V>, dim3((unsigned)blocks, (unsigned)((a.nvy + a.Q - 1) / a.Q)),
+  VLP4D_CUDA_TRY(launch_dep(c, k_v_cols<T, DVX, DVY, V>, dim3((unsigned)blocks, (unsigned)((a.nvy + a.Q - 1) / a.Q)),
                             dim3(kVColsThreads), 0, s, a));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;

@@ -200,6 +200,7 @@ __device__ __forceinline__ void sweep_y_pairs(const double *src, int nx, int h, 
 // for the whole kernel; blockDim = (nx/4) * (R/RT).
 template <typename T, int NX, int RT, bool DX, bool DY, bool RHO, bool INPLACE = false>
 __global__ void __launch_bounds__(512) k_plane(PlaneArgs a) {
+  pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem[];
   const int nx = NX ? NX : a.nx;
@@ -647,6 +648,7 @@ __device__ __forceinline__ int xyxy_swz(int chunk) { return chunk ^ ((chunk >> 3
 // stencils has no use for one).
 template <typename T, int NX, int RT, bool X8 = false, bool RHO = true>
 __global__ void __launch_bounds__(512) k_plane_xyxy(PlaneArgs a) {
+  pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem[];
   const int nx = NX ? NX : a.nx;
@@ -886,6 +888,7 @@ __device__ __forceinline__ void x11_pair_row(const double *row, int a0, int nx, 
 
 template <int NX, int RT, bool RHO = true>
 __global__ void __launch_bounds__(512) k_plane_xyxy64(PlaneArgs a) {
+  pdl_wait();
   pdl_trigger();
   using T = double;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -1160,7 +1163,7 @@ int run_plane(vlp4d_ctx *c, const PlaneArgs &args, PlaneCfg &cfg, cudaStream_t s
   if (RHO && G > c->rho_part_groups) G = c->rho_part_groups;
   cfg.G = (int)G;
   cfg.grid = (int)G * cfg.cpp;
-  kern<<<cfg.grid, cfg.threads, cfg.smem, s>>>(args);
+  VLP4D_CUDA_TRY(launch_dep(c, kern, dim3(cfg.grid), dim3(cfg.threads), cfg.smem, s, args));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }
@@ -1270,7 +1273,7 @@ int run_xyxy(vlp4d_ctx *c, const PlaneArgs &args, PlaneCfg &cfg, bool rho, cudaS
   if (G > c->rho_part_groups) G = c->rho_part_groups;
   cfg.G = (int)G;
   cfg.grid = (int)G * cfg.cpp;
-  kern<<<cfg.grid, cfg.threads, cfg.smem, s>>>(args);
+  VLP4D_CUDA_TRY(launch_dep(c, kern, dim3(cfg.grid), dim3(cfg.threads), cfg.smem, s, args));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }
@@ -1365,7 +1368,7 @@ int run_xyxy64(vlp4d_ctx *c, PlaneArgs args, PlaneCfg &cfg, bool rho, cudaStream
   if (G > c->rho_part_groups) G = c->rho_part_groups;
   cfg.G = (int)G;
   cfg.grid = (int)G * cfg.cpp;
-  kern<<<cfg.grid, cfg.threads, cfg.smem, s>>>(args);
+  VLP4D_CUDA_TRY(launch_dep(c, kern, dim3(cfg.grid), dim3(cfg.threads), cfg.smem, s, args));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }

@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(512) k_vslab(const __grid_constant__ CUtensorM
     mbar_fence_init();
   }
   pdl_wait();
+  pdl_trigger();
   __syncthreads();
 
   // Look-ahead cursor: slab S of the sequence (the first S are issued here).
@@ -457,7 +458,7 @@ int run_vslab(vlp4d_ctx *c, const CUtensorMap &map, const VslabArgs &args, const
   if (cap > 0 && per_sm > cap) per_sm = cap;
   long long grid = (long long)per_sm * c->num_sms;
   if (grid > args.nitems) grid = args.nitems;
-  VLP4D_CUDA_TRY(launch_pdl(kern, dim3((unsigned)grid), dim3(cfg.threads), cfg.smem, s, map, args));
+  VLP4D_CUDA_TRY(launch_dep(c, kern, dim3((unsigned)grid), dim3(cfg.threads), cfg.smem, s, map, args));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }

@@ -291,7 +291,7 @@ int launch_rho_finish(vlp4d_ctx *c, int groups, cudaStream_t s) {
   const long long nxy = c->g.nxy();
   const bool wide = moment_wide(groups);
   const int cells = wide ? 16 : 32;
-  VLP4D_CUDA_TRY(launch_pdl(wide ? k_rho_finish<16> : k_rho_finish<32>, dim3((unsigned)((nxy + cells - 1) / cells)),
+  VLP4D_CUDA_TRY(launch_dep(c, wide ? k_rho_finish<16> : k_rho_finish<32>, dim3((unsigned)((nxy + cells - 1) / cells)),
                             dim3(kMomentThreads), 0, s, c->rho_part, c->rho, nxy, groups, c->g.dx[2], c->g.dx[3]));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
@@ -335,7 +335,7 @@ int launch_field_poisson(vlp4d_ctx *c, cudaStream_t s) {
 }
 
 int launch_diags(vlp4d_ctx *c, int iter, cudaStream_t s) {
-  VLP4D_CUDA_TRY(launch_pdl(k_diags, dim3(1), dim3(1024), 0, s, c->rho, c->ex, c->ey, c->g.nxy(), c->g.dx[0], c->g.dx[1],
+  VLP4D_CUDA_TRY(launch_dep(c, k_diags, dim3(1), dim3(1024), 0, s, c->rho, c->ex, c->ey, c->g.nxy(), c->g.dx[0], c->g.dx[1],
                             c->nrj, c->mass, c->nrjx, c->nrjy, iter));
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
@@ -354,6 +354,7 @@ int diags_async(vlp4d_ctx *c, int iter, cudaStream_t s) {
 
 int diags_join(vlp4d_ctx *c, cudaStream_t s) {
   VLP4D_CUDA_TRY(cudaStreamWaitEvent(s, c->ev_join, 0));
+  c->after_event = true;
   return VLP4D_OK;
 }
 

@@ -52,7 +52,7 @@ void count_launch();
 
 // Programmatic dependent launch along a step's chain of small kernels
 // (moment -> field solve -> v tables -> v pass): a kernel launched with
-// launch_pdl may start while the one before it in the stream still runs, and
+// launch_dep may start while the one before it in the stream still runs, and
 // calls pdl_wait before it touches global memory; the one before calls
 // pdl_trigger once it has itself passed its wait, so at most two kernels
 // overlap.  What the predecessor writes is read with plain or L2 loads only
@@ -62,21 +62,6 @@ void count_launch();
 // steps: 1232 -> 1201 us.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr = {};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
-}
 
 // Geometry of one run, in the reference's Domain terms.
 struct Grid {
@@ -199,10 +184,32 @@ struct vlp4d_ctx {
   // before rho is next written), overlapping the v-table build and the vx/vy
   // pass.
   cudaStream_t side = nullptr;
+  // Set by diags_join: the next launch_dep follows an event in its stream and
+  // is an ordinary launch.
+  bool after_event = false;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 };
 
 namespace vlp4d {
+
+// A launch that depends programmatically on the kernel before it in its
+// stream, or an ordinary one where an event came between.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dep(vlp4d_ctx *c, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                       Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = c->after_event ? 0 : 1;
+  c->after_event = false;
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
 
 // Error-word bits (vlp4d_check): a bounded wait ran out; a vlp4d_mpi foot
 // left its interpolation range; a slab's vy sweep needed planes beyond its
