@@ -232,6 +232,9 @@ __global__ void __launch_bounds__(512) k_plane(PlaneArgs a) {
   const int r0 = rg * RT;
 
   const int chunk = blockIdx.x % a.cpp;
+  // First output row; the last chunk of a height that does not divide ny
+  // overlaps the one before (both store the same values there).
+  const int row0 = chunk * R < ny - R ? chunk * R : ny - R;
   const int G = gridDim.x / a.cpp;
   const int g = blockIdx.x / a.cpp;
   const long long planes = (long long)a.nvx * a.nvy;
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(512) k_plane(PlaneArgs a) {
   // Thread 0: stage the input rows of item `it` into its slot.
   auto issue = [&](long long it) {
     const long long p = g + it * G;
-    int phys = chunk * R;
+    int phys = row0;
     if (DY) {
       phys += yrec[(int)(p / a.nvx)].m;
       if (phys >= ny) phys -= ny;
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(512) k_plane(PlaneArgs a) {
     const bool ok = mbar_wait_bounded(&bars[slot], parity);
     const long long p = g + it * G;
     const T *in = slots + (size_t)slot * slot_elems;
-    T *outp = static_cast<T *>(a.fout) + p * plane_elems + (long long)chunk * R * nx;
+    T *outp = static_cast<T *>(a.fout) + p * plane_elems + (long long)row0 * nx;
     T *xs = xs_base + (size_t)(it & 1) * slot_elems;
 
     if (DX) {  // Phase X: staged rows rg, rg+RG, ...; this thread's column quad.
@@ -444,7 +447,7 @@ __global__ void __launch_bounds__(512) k_plane(PlaneArgs a) {
     if (threadIdx.x == 0 && it + S < n_items) issue(it + S);
   }
   if (RHO) {
-    double *dst = a.rho_part + (long long)g * plane_elems + ((long long)chunk * R + r0) * nx + (PAIRS ? yc : c0);
+    double *dst = a.rho_part + (long long)g * plane_elems + ((long long)row0 + r0) * nx + (PAIRS ? yc : c0);
     const int second = PAIRS ? hx : 2;  // element offset of the second double pair
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
@@ -667,6 +670,9 @@ __global__ void __launch_bounds__(512) k_plane_xyxy(PlaneArgs a) {
   const int c0 = cg * 4;
   const int r0 = rg * RT;
   const int chunk = blockIdx.x % a.cpp;
+  // First output row; the last chunk of a height that does not divide ny
+  // overlaps the one before (both store the same values there).
+  const int row0 = chunk * R < ny - R ? chunk * R : ny - R;
   const int G = gridDim.x / a.cpp;
   const int g = blockIdx.x / a.cpp;
   const long long planes = (long long)a.nvx * a.nvy;
@@ -683,7 +689,7 @@ __global__ void __launch_bounds__(512) k_plane_xyxy(PlaneArgs a) {
 
   auto issue = [&](long long it) {
     const long long p = g + it * G;
-    int phys = (chunk * R + yrec[(int)(p / a.nvx)].m) % ny;
+    int phys = (row0 + yrec[(int)(p / a.nvx)].m) % ny;
     uint64_t *bar = &bars[it % S];
     mbar_arrive_expect_tx(bar, slot_bytes);
     const T *src = static_cast<const T *>(a.fin) + p * plane_elems;
@@ -720,7 +726,7 @@ __global__ void __launch_bounds__(512) k_plane_xyxy(PlaneArgs a) {
     const long long p = g + it * G;
     const T *in = slots + (size_t)slot * slot_elems;
     T *ys = ys_base + (size_t)(it & 1) * R * nx;
-    T *outp = static_cast<T *>(a.fout) + p * plane_elems + (long long)chunk * R * nx;
+    T *outp = static_cast<T *>(a.fout) + p * plane_elems + (long long)row0 * nx;
     {  // Y11: rows r0 .. r0+RT-1 of this thread's column quad.
       W11<T> wy;
       read_line11(yrec[ivy], wy);
@@ -820,7 +826,7 @@ __global__ void __launch_bounds__(512) k_plane_xyxy(PlaneArgs a) {
   if constexpr (!RHO) {
     return;
   } else if constexpr (X8) {
-    double *rdst = a.rho_part + (long long)g * plane_elems + ((long long)chunk * R + r8) * nx + c8;
+    double *rdst = a.rho_part + (long long)g * plane_elems + ((long long)row0 + r8) * nx + c8;
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -830,7 +836,7 @@ __global__ void __launch_bounds__(512) k_plane_xyxy(PlaneArgs a) {
         p2[1] = make_double2(racc[2 * i + h][2], racc[2 * i + h][3]);
       }
   } else {
-    double *rdst = a.rho_part + (long long)g * plane_elems + ((long long)chunk * R + r0) * nx + c0;
+    double *rdst = a.rho_part + (long long)g * plane_elems + ((long long)row0 + r0) * nx + c0;
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       reinterpret_cast<double2 *>(rdst + (size_t)i * nx)[0] = make_double2(racc[i][0], racc[i][1]);
@@ -886,7 +892,7 @@ __device__ __forceinline__ void x11_pair_row(const double *row, int a0, int nx, 
   else x11_pair_from<0>(t, w, o);
 }
 
-template <int NX, int RT, bool RHO = true>
+template <int NX, int RT, bool RHO, bool OVER>
 __global__ void __launch_bounds__(512) k_plane_xyxy64(PlaneArgs a) {
   pdl_wait();
   pdl_trigger();
@@ -910,6 +916,9 @@ __global__ void __launch_bounds__(512) k_plane_xyxy64(PlaneArgs a) {
   const int yc = cg * 2;  // Y11 and the moment: columns yc, yc+1 and yc+nx/2, yc+nx/2+1
   const int r0 = rg * RT;
   const int chunk = blockIdx.x % a.cpp;
+  // OVER: the last chunk, whose height does not divide ny, overlaps the one
+  // before (both store the same values there).
+  const int shift = OVER && (chunk + 1) * R > ny ? (chunk + 1) * R - ny : 0;
   const int G = gridDim.x / a.cpp;
   const int g = blockIdx.x / a.cpp;
   const long long planes = (long long)a.nvx * a.nvy;
@@ -926,7 +935,7 @@ __global__ void __launch_bounds__(512) k_plane_xyxy64(PlaneArgs a) {
 
   auto issue = [&](long long it) {
     const long long p = g + it * G;
-    int phys = (chunk * R + yrec[(int)(p / a.nvx)].m) % ny;
+    int phys = (chunk * R - shift + yrec[(int)(p / a.nvx)].m) % ny;
     uint64_t *bar = &bars[it % S];
     mbar_arrive_expect_tx(bar, slot_bytes);
     const T *src = static_cast<const T *>(a.fin) + p * plane_elems;
@@ -966,7 +975,7 @@ __global__ void __launch_bounds__(512) k_plane_xyxy64(PlaneArgs a) {
     const bool ok = mbar_wait_bounded(&bars[slot], parity);
     const long long p = g + it * G;
     T *in = slots + (size_t)slot * slot_elems;
-    T *outp = static_cast<T *>(a.fout) + p * plane_elems + (long long)chunk * R * nx;
+    T *outp = static_cast<T *>(a.fout) + p * plane_elems + ((long long)chunk * R - shift) * nx;
     {  // X11 in place on the staged rows rg, rg + RG, ... (this warp's rows),
        // output pairs at columns yc and yc + nx/2 (16-byte accesses,
        // consecutive across the lanes).
@@ -1049,7 +1058,7 @@ __global__ void __launch_bounds__(512) k_plane_xyxy64(PlaneArgs a) {
     }
   }
   if constexpr (RHO) {
-    double *rdst = a.rho_part + (long long)g * plane_elems + ((long long)chunk * R + r0) * nx + yc;
+    double *rdst = a.rho_part + (long long)g * plane_elems + ((long long)chunk * R - shift + r0) * nx + yc;
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       *reinterpret_cast<double2 *>(rdst + (size_t)i * nx) = make_double2(racc[i][0], racc[i][1]);
@@ -1082,6 +1091,29 @@ size_t plane_smem(int R, int halo, int nx, size_t elem, int stages, bool dx, boo
   const size_t slot = (size_t)(R + halo) * nx * elem;
   const size_t rec = elem == 4 ? 32 : 64;
   return kBarBytes + rec * ((dx ? nvx : 0) + (dy ? nvy : 0)) + stages * slot + ((dx && dy && !inplace) ? 2 * slot : 0);
+}
+
+// Chunk height that need not divide ny (the last chunk overlaps the one
+// before): the multiple of four up to rmax rows with the fewest rows swept,
+// chunks x (R + halo), whose block and shared memory fit; 0: none.  Taken
+// where the tallest divisor is short or no multiple of four, so that a thread
+// has one row instead of four (us, divisor against overlap: 64 x 55 x 48 x 50,
+// 11 rows: x and y FP64 47.9 / 30.6, FP32 27.1 / 17.2; 72 x 55 x 64 x 64 FP32 60.0 /
+// 33.3; 80 x 90 x 72 x 70, 18 rows, FP64 242 / 146; five steps of 64 x 74 x 48 x 50,
+// two rows, FP32 754 / 449, FP64 1341 / 619).
+template <typename Fits>
+int overlap_rows(int ny, int rmax, int halo, int ncg, Fits fits) {
+  int best = 0;
+  long long cost = 0;
+  for (int r = rmax < ny ? rmax / 4 * 4 : ny / 4 * 4; r >= 8; r -= 4) {
+    if (ncg * (r / 4) > 512 || ncg * (r / 4) < 32 || !fits(r)) continue;
+    const long long k = (long long)((ny + r - 1) / r) * (r + halo);
+    if (!best || k < cost) {
+      best = r;
+      cost = k;
+    }
+  }
+  return best;
 }
 
 // Chooses the chunk height R, rows per thread RT, the pipeline depth and the
@@ -1119,6 +1151,15 @@ bool plane_config(const vlp4d_ctx *c, bool dx, bool dy, PlaneCfg &cfg) {
     rt = t;
     break;
   }
+  if (!forced_r && !forced_rt && (!R || rt != 4 || R < 16)) {
+    const int r = overlap_rows(ny, rmax, halo, ncg, [&](int q) {
+      return plane_smem(q, halo, nx, elem, 2, dx, dy, c->g.n[2], c->g.n[3], inplace) <= 224 * 1024;
+    });
+    if (r) {
+      R = r;
+      rt = 4;
+    }
+  }
   if (!R) return false;
   const size_t two_per_sm = 112 * 1024, one_per_sm = 224 * 1024;
   int stages = 0;
@@ -1130,12 +1171,13 @@ bool plane_config(const vlp4d_ctx *c, bool dx, bool dy, PlaneCfg &cfg) {
     if (!stages) stages = 3;
   }
   if (stages < 2 || stages > kMaxStages) return false;
+  if (!forced_s && plane_smem(R, halo, nx, elem, stages, dx, dy, c->g.n[2], c->g.n[3], inplace) > one_per_sm) stages = 2;
   const size_t smem = plane_smem(R, halo, nx, elem, stages, dx, dy, c->g.n[2], c->g.n[3], inplace);
   if (smem > one_per_sm) return false;
   cfg.R = R;
   cfg.rt = rt;
   cfg.stages = stages;
-  cfg.cpp = ny / R;
+  cfg.cpp = (ny + R - 1) / R;
   cfg.threads = ncg * (R / rt);
   cfg.smem = smem;
   cfg.inplace = inplace;
@@ -1242,8 +1284,19 @@ bool xyxy_config(const vlp4d_ctx *c, PlaneCfg &cfg) {
     cfg.rt = t;
     cfg.stages = st;
   }
+  if (!forced && !forced_r && c->elem == 4 && (!cfg.R || cfg.rt != 4 || cfg.R < 16)) {
+    auto stages = [&](int q) { return xyxy_smem(q, nx, c->elem, 3, c->g.n[2], c->g.n[3]) <= 112 * 1024 ? 3 : 2; };
+    const int r = overlap_rows(ny, 32, 10, ncg, [&](int q) {
+      return xyxy_smem(q, nx, c->elem, stages(q), c->g.n[2], c->g.n[3]) <= 224 * 1024;
+    });
+    if (r) {
+      cfg.R = r;
+      cfg.rt = 4;
+      cfg.stages = stages(r);
+    }
+  }
   if (!cfg.R) return false;
-  cfg.cpp = ny / cfg.R;
+  cfg.cpp = (ny + cfg.R - 1) / cfg.R;
   cfg.threads = ncg * (cfg.R / cfg.rt);
   cfg.smem = xyxy_smem(cfg.R, nx, c->elem, cfg.stages, c->g.n[2], c->g.n[3]);
   return true;
@@ -1314,35 +1367,50 @@ bool xyxy64_config(const vlp4d_ctx *c, PlaneCfg &cfg) {
   if (forced && (forced < 2 || forced > kMaxStages)) return false;
   const int forced_r = env_int("VLP4D_XYXY64_R", 0);  // chunk height, for tuning sweeps
   const int rmax = forced_r > 0 ? forced_r : 64;
+  auto depth = [&](int r) {
+    int st = forced ? forced : 2;
+    if (!forced && xyxy64_smem(r, nx, 2, c->g.n[2], c->g.n[3]) > 112 * 1024 &&
+        xyxy64_smem(r, nx, 3, c->g.n[2], c->g.n[3]) <= 224 * 1024)
+      st = 3;
+    return st;
+  };
+  bool found = false;
   for (int r = ny < rmax ? ny : rmax; r >= 1; --r) {
     if (ny % r) continue;
     if (forced_r && r != forced_r) continue;
     const int t = r % 4 == 0 ? 4 : 1;
     const int threads = ncg * (r / t);
     if (threads > 512) continue;
-    int st = forced ? forced : 2;
-    if (!forced && xyxy64_smem(r, nx, 2, c->g.n[2], c->g.n[3]) > 112 * 1024 &&
-        xyxy64_smem(r, nx, 3, c->g.n[2], c->g.n[3]) <= 224 * 1024)
-      st = 3;
-    const size_t smem = xyxy64_smem(r, nx, st, c->g.n[2], c->g.n[3]);
-    if (smem > 224 * 1024) continue;
+    if (xyxy64_smem(r, nx, depth(r), c->g.n[2], c->g.n[3]) > 224 * 1024) continue;
     cfg.R = r;
     cfg.rt = t;
-    cfg.stages = st;
-    cfg.cpp = ny / r;
-    cfg.threads = threads;
-    cfg.smem = smem;
-    return true;
+    found = true;
+    break;
   }
-  return false;
+  if (!forced && !forced_r && (!found || cfg.rt != 4 || cfg.R < 16)) {
+    const int r = overlap_rows(ny, 64, 10, ncg, [&](int q) {
+      return xyxy64_smem(q, nx, depth(q), c->g.n[2], c->g.n[3]) <= 224 * 1024;
+    });
+    if (r) {
+      cfg.R = r;
+      cfg.rt = 4;
+      found = true;
+    }
+  }
+  if (!found) return false;
+  cfg.stages = depth(cfg.R);
+  cfg.cpp = (ny + cfg.R - 1) / cfg.R;
+  cfg.threads = ncg * (cfg.R / cfg.rt);
+  cfg.smem = xyxy64_smem(cfg.R, nx, cfg.stages, c->g.n[2], c->g.n[3]);
+  return true;
 }
 
 }  // namespace
 
-// Chunks of fewer than five rows (ny without such a divisor) sweep ten halo
-// rows each along x: two passes are faster (five steps, 64 x 74 x 48 x 50 in
-// chunks of two: 1.34 ms joined, 1.10 in two passes; 64 x 49 in seven: 0.76 /
-// 0.80).
+// Chunks of fewer than five rows sweep ten halo rows each along x: two passes
+// are faster (five steps, 64 x 74 x 48 x 50 in chunks of two: 1.34 ms joined,
+// 1.10 in two passes; 64 x 49 in seven: 0.76 / 0.80).  Only where overlap_rows
+// finds nothing.
 bool xyxy64_available(const vlp4d_ctx *c) {
   PlaneCfg cfg;
   return c->fused && xyxy64_config(c, cfg) && (cfg.R >= 5 || cfg.R == c->g.n[1]);
@@ -1352,7 +1420,12 @@ namespace {
 
 template <int NX, int RT>
 int run_xyxy64(vlp4d_ctx *c, PlaneArgs args, PlaneCfg &cfg, bool rho, cudaStream_t s) {
-  auto kern = rho ? k_plane_xyxy64<NX, RT, true> : k_plane_xyxy64<NX, RT, false>;
+  // The last chunk overlaps where the height does not divide ny.  (A kernel of
+  // its own, and 64-bit row offsets there: with one 32-bit offset for all uses
+  // the 128^4 pass took 1.12 ms instead of 1.04.)
+  const bool over = c->g.n[1] % cfg.R != 0;
+  auto kern = over ? (rho ? k_plane_xyxy64<NX, RT, true, true> : k_plane_xyxy64<NX, RT, false, true>)
+                   : (rho ? k_plane_xyxy64<NX, RT, true, false> : k_plane_xyxy64<NX, RT, false, false>);
   VLP4D_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem));
   int per_sm = 0;
   VLP4D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, cfg.threads, cfg.smem));
@@ -1417,11 +1490,11 @@ int launch_advect_xy(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTabl
   PlaneCfg cfg;
   if (!plane_config(c, do_x, do_y, cfg)) return VLP4D_ERR_UNSUPPORTED;
   // Where the column kernel (launch_xy_cols) is faster, decline: chunks of a
-  // few rows (ny without a divisor up to 32: 64 x 74 rows in pairs, x and y,
-  // FP64 107 against 66 us, FP32 66 against 57; chunks of 7 rows: 45.7 / 43.9 and
-  // 27.1 / 37.5), and in FP64 one row per thread outside the in-place form (72 x
-  // 60 in chunks of 30: 168 / 155 us, 80 x 90 in 18: 242 / 154; four rows per
-  // thread, 100 x 100 in 20: 82 / 104).
+  // few rows (64 x 74 rows in pairs, x and y, FP64 107 against 66 us, FP32 66
+  // against 57; chunks of 7 rows: 45.7 / 43.9 and 27.1 / 37.5), and in FP64 one row
+  // per thread outside the in-place form (72 x 60 in chunks of 30: 168 / 155 us,
+  // 80 x 90 in 18: 242 / 154; four rows per thread, 100 x 100 in 20: 82 / 104).
+  // Both are left only where overlap_rows finds nothing.
   if (!c->fused_only && do_x && do_y &&
       (cfg.R < 5 && cfg.R < c->g.n[1] || (c->elem == 8 && !cfg.inplace && cfg.rt == 1)))
     return VLP4D_ERR_UNSUPPORTED;

@@ -90,3 +90,29 @@ def test_uneven_vy_segments(pkg, cuda, monkeypatch, n, dtype):
             getattr(gen, name)(f, want, 0.2)
             fz.check()
             assert float((out - want).abs().max()) <= tol * float(want.abs().max()), name
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("n", [(64, 37, 8, 9), (32, 74, 8, 8), (72, 55, 8, 8), (128, 127, 8, 8), (20, 21, 8, 8), (256, 13, 8, 8)])
+def test_overlapping_row_chunks(pkg, cuda, monkeypatch, n, dtype):
+    """The plane passes where the chunk height does not divide ny (the last
+    chunk overlaps the one before), forced, against one thread per output, and
+    the joined pass against two passes; tolerances as for the other shapes."""
+    torch = cuda
+    tol = 1e-14 if dtype == "f64" else 2e-7
+    with _ctx(pkg, monkeypatch, n, dtype, "fused") as fz, _ctx(pkg, monkeypatch, n, dtype, "generic") as gen:
+        f = fz.empty_f()
+        fz.init_case(f)
+        for name in ("advect_x", "advect_y", "advect_xy", "advect_xy_moment"):
+            out, want = (torch.full_like(f, 9.0) for _ in range(2))
+            getattr(fz, name)(f, out, 0.21)
+            getattr(gen, name)(f, want, 0.21)
+            fz.check()
+            assert float((out - want).abs().max()) <= tol * float(want.abs().max()), name
+        assert float((fz.rho - gen.rho).abs().max()) <= (1e-13 if dtype == "f64" else 1e-6) * float(gen.rho.abs().max())
+        out, half, want = (torch.full_like(f, 9.0) for _ in range(3))
+        fz.advect_xyxy(f, out, 0.21)
+        fz.advect_xy(f, half, 0.21)
+        fz.advect_xy_moment(half, want, 0.21)
+        fz.check()
+        assert float((out - want).abs().max()) <= (1e-13 if dtype == "f64" else 2e-6) * float(want.abs().max())
