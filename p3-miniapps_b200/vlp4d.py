@@ -231,12 +231,30 @@ class _DevArray:
                                          "version": 3, "strides": None}
 
 
-def _stream_ptr(stream) -> Optional[int]:
+def _bind_current_stream():
+    """The handle of PyTorch's current stream on the current device, without
+    building a torch.cuda.Stream for every call (3.4 us, of 7 to 9 us that a
+    small call takes on the host, against 0.1)."""
     import torch
 
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return stream.cuda_stream
+    torch.cuda.current_stream()  # initialises CUDA
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    device = getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or device is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
+
+
+_current_stream = None
+
+
+def _stream_ptr(stream) -> Optional[int]:
+    global _current_stream
+    if stream is not None:
+        return stream.cuda_stream
+    if _current_stream is None:
+        _current_stream = _bind_current_stream()
+    return _current_stream()
 
 
 class Context:

@@ -43,3 +43,16 @@ def test_moment(pkg, cuda, n, dtype):
         want = f.double().sum((0, 1)) * dom.dx[2] * dom.dx[3]
         # At most 2 nv roundings of sums below nv.
         assert float((ctx.rho - want).abs().max()) <= 2 * 1.2e-16 * (n[2] * n[3]) ** 2 * dom.dx[2] * dom.dx[3] + 1e-16
+
+
+def test_calls_go_to_the_current_stream(pkg, cuda):
+    """Without a stream argument a call runs on PyTorch's current stream, the
+    default one, a side stream and the default one again."""
+    torch = cuda
+    ptr = pkg.vlp4d._stream_ptr
+    side = torch.cuda.Stream()
+    assert ptr(None) == torch.cuda.current_stream().cuda_stream
+    with torch.cuda.stream(side):
+        assert ptr(None) == side.cuda_stream
+    assert ptr(None) == torch.cuda.current_stream().cuda_stream
+    assert ptr(side) == side.cuda_stream
