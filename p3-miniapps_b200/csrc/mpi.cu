@@ -763,21 +763,19 @@ namespace {
 // 4x4 spline interpolation of the coefficients in tmp at
 // (x - dt vx, y - dt vy).  A foot outside [xmin-1, xmax] (in cells) sets
 // bit 2 of *err and the point receives 0.
-__global__ void k_mpi_advect_2d(const double *__restrict__ tmp, double *__restrict__ fn, HGrid h, double dt,
-                                int *__restrict__ err) {
-  const long long cells = (long long)h.n[0] * h.n[1] * h.n[2] * h.n[3];
+// Block (32 x, 8 y) of (ix, iy), a thread takes the planes p = z, z + G, ...
+// (48 x 44 x 40 x 36: 37 us; one thread per cell with its index taken apart by
+// 64-bit divisions, 45 us.)
+__global__ void __launch_bounds__(256) k_mpi_advect_2d(const double *__restrict__ tmp, double *__restrict__ fn,
+                                                       HGrid h, double dt, int *__restrict__ err) {
+  const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y;
+  if (ix >= h.n[0] || iy >= h.n[1]) return;
+  const int planes = h.n[2] * h.n[3];
+  const double x = add(h.minp[0], mul((double)ix, h.dx[0]));
+  const double y = add(h.minp[1], mul((double)iy, h.dx[1]));
   bool bad = false;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cells;
-       i += (long long)gridDim.x * blockDim.x) {
-    long long r = i;
-    const int ix = (int)(r % h.n[0]);
-    r /= h.n[0];
-    const int iy = (int)(r % h.n[1]);
-    r /= h.n[1];
-    const int ivx = (int)(r % h.n[2]);
-    const int ivy = (int)(r / h.n[2]);
-    const double x = add(h.minp[0], mul((double)ix, h.dx[0]));
-    const double y = add(h.minp[1], mul((double)iy, h.dx[1]));
+  for (int p = blockIdx.z; p < planes; p += gridDim.z) {
+    const int ivy = p / h.n[2], ivx = p - ivy * h.n[2];
     const double vx = add(h.minp[2], mul((double)ivx, h.dx[2]));
     const double vy = add(h.minp[3], mul((double)ivy, h.dx[3]));
     const double fx = mul(sub(sub(x, mul(dt, vx)), h.minp[0]), h.inv_dx[0]);
@@ -787,13 +785,19 @@ __global__ void k_mpi_advect_2d(const double *__restrict__ tmp, double *__restri
     if (i0 < -1 || i0 > h.n[0] - 1 || i1 < -1 || i1 > h.n[1] - 1) {
       bad = true;
     } else {
-      double ex[4], ey[4];
+      double ex[4], ey[4], t[4][4];
+      const double *row = tmp + h.at(i0 - 1, i1 - 1, ivx, ivy);
+#pragma unroll
+      for (int ky = 0; ky < 4; ++ky)
+#pragma unroll
+        for (int kx = 0; kx < 4; ++kx) t[ky][kx] = __ldg(row + ky * h.s[1] + kx);
       bspline_w<true>(sub(fx, (double)i0), ex);
       bspline_w<true>(sub(fy, (double)i1), ey);
+#pragma unroll
       for (int ky = 0; ky < 4; ++ky) {
-        const double *row = tmp + h.at(i0 - 1, i1 - 1 + ky, ivx, ivy);
         double s = 0.;
-        for (int kx = 0; kx < 4; ++kx) s = add(s, mul(ex[kx], row[kx]));
+#pragma unroll
+        for (int kx = 0; kx < 4; ++kx) s = add(s, mul(ex[kx], t[ky][kx]));
         v = add(v, mul(ey[ky], s));
       }
     }
@@ -1472,8 +1476,35 @@ __global__ void k_mpi_rho_partial(const double *__restrict__ f, double *__restri
   const int ix = (int)(ixy % h.n[0]), iy = (int)(ixy / h.n[0]);
   const long long nv = (long long)h.n[2] * h.n[3];
   const long long v0 = nv * g / groups, v1 = nv * (g + 1) / groups;
+  // Eight planes' loads ahead of their sums; the planes follow one another
+  // without divisions.
   double s = 0.;
-  for (long long v = v0; v < v1; ++v) s += __ldg(f + h.at(ix, iy, (int)(v % h.n[2]), (int)(v / h.n[2])));
+  int ivx = (int)(v0 % h.n[2]);
+  const double *p = f + h.at(ix, iy, ivx, (int)(v0 / h.n[2]));
+  const long long row = h.s[3] - (long long)(h.n[2] - 1) * h.s[2];  // from the last vx to the next vy
+  auto next = [&] {
+    if (++ivx == h.n[2]) {
+      ivx = 0;
+      p += row;
+    } else {
+      p += h.s[2];
+    }
+  };
+  long long v = v0;
+  for (; v + 8 <= v1; v += 8) {
+    double t[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      t[k] = __ldg(p);
+      next();
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += t[k];
+  }
+  for (; v < v1; ++v) {
+    s += __ldg(p);
+    next();
+  }
   part[(long long)g * nxy + ixy] = s;
 }
 
@@ -1490,26 +1521,46 @@ __global__ void __launch_bounds__(256) k_mpi_l2_partial(const double *__restrict
                                                         double *__restrict__ l2) {
   // A warp walks rows (32 x positions at a time); the block's 8 warps take
   // rows r = 8 * blockIdx + warp, stepping by 8 * gridDim.
-  const long long rows = (long long)h.n[1] * h.n[2] * h.n[3];
+  const long long rows = (long long)h.n[1] * h.n[2] * h.n[3];  // below 2^32: such an array would be 550 GB
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double s = 0., cp = 0.;
-  for (long long r = (long long)blockIdx.x * nw + warp; r < rows; r += (long long)gridDim.x * nw) {
-    const int iy = (int)(r % h.n[1]);
-    const long long rv = r / h.n[1];
-    const double *row = f + h.at(0, iy, (int)(rv % h.n[2]), (int)(rv / h.n[2]));
+  // Four rows' loads at a time ahead of their sums.
+  const long long step = (long long)gridDim.x * nw;
+  for (long long r = (long long)blockIdx.x * nw + warp; r < rows; r += 4 * step) {
+    const double *row[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned q = (unsigned)(r + k * step < rows ? r + k * step : r);
+      const unsigned rv = q / (unsigned)h.n[1], ivy = rv / (unsigned)h.n[2];
+      row[k] = f + h.at(0, (int)(q - rv * h.n[1]), (int)(rv - ivy * h.n[2]), (int)ivy);
+    }
+    const int live = rows - r > 3 * step ? 4 : (int)((rows - r + step - 1) / step);
     for (int ix = lane; ix < h.n[0]; ix += 32) {
-      const double v = __ldg(row + ix);
-      kahan(s, cp, v * v);
+      double v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = __ldg(row[k] + ix);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k < live) kahan(s, cp, v[k] * v[k]);
     }
   }
   __shared__ double ws[256];
   ws[threadIdx.x] = s - cp;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  // The first warp: eight threads' sums per lane, then the lanes', in order.
+  if (threadIdx.x < 32) {
     double a = 0., b = 0.;
-    for (int t = 0; t < (int)blockDim.x; ++t) kahan(a, b, ws[t]);
-    l2[2 * blockIdx.x] = a;
-    l2[2 * blockIdx.x + 1] = b;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) kahan(a, b, ws[threadIdx.x * 8 + t]);
+    double A = 0., B = 0.;
+    for (int l = 0; l < 32; ++l) {
+      kahan(A, B, __shfl_sync(0xffffffffu, a, l));
+      kahan(A, B, -__shfl_sync(0xffffffffu, b, l));
+    }
+    if (threadIdx.x == 0) {
+      l2[2 * blockIdx.x] = A;
+      l2[2 * blockIdx.x + 1] = B;
+    }
   }
 }
 
@@ -1881,7 +1932,12 @@ int vlp4d_mpi_advect_2d(vlp4d_ctx *ctx, void *fn, void *fn_tmp, double dt, void 
   const HGrid h = make_hgrid(ctx);
   cudaStream_t s = (cudaStream_t)stream;
   VLP4D_CUDA_TRY(cudaMemcpyAsync(fn_tmp, fn, sizeof(double) * (size_t)h.total(), cudaMemcpyDeviceToDevice, s));
-  k_mpi_advect_2d<<<ctx->num_sms * 8, 256, 0, s>>>((const double *)fn_tmp, (double *)fn, h, dt, ctx->d_err);
+  const dim3 grid((unsigned)((h.n[0] + 31) / 32), (unsigned)((h.n[1] + 7) / 8));
+  long long G = ((long long)ctx->num_sms * 16 + (long long)grid.x * grid.y - 1) / ((long long)grid.x * grid.y);
+  const long long planes = (long long)h.n[2] * h.n[3];
+  if (G > planes) G = planes;
+  k_mpi_advect_2d<<<dim3(grid.x, grid.y, (unsigned)G), dim3(32, 8), 0, s>>>((const double *)fn_tmp, (double *)fn, h, dt,
+                                                                            ctx->d_err);
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }
