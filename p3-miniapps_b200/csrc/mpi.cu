@@ -48,7 +48,7 @@ struct HGrid {
   int n[4];
   long long e[4];  // n + 6
   long long s[4];  // strides: 1, e0, e0 e1, e0 e1 e2
-  int is[4];       // the same strides as int (an array has fewer than 2^31 elements)
+  int is[4];       // the same strides as int (a stride of 2^31 would be an array of 270 GB)
   double minp[4], maxp[4], dx[4], inv_dx[4];
   // Admissible feet of the 4D advection (Advection.hpp thrust :249-250):
   // [min + local_min*h - h, min + local_max*h + h] with local = 0..n-1.
@@ -89,6 +89,8 @@ HGrid make_hgrid(const vlp4d_ctx *c) {
 }
 
 __device__ __forceinline__ int wrapi(int i, int n) { return ((i % n) + n) % n; }
+// The same for i in [-n, 2 n).
+__device__ __forceinline__ int wrap1(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 
 // Separately rounded arithmetic (the reference's x86-64 build has no FMA).
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
@@ -125,7 +127,9 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // one; B of two and one a thread per point; B empty a copy.  One thread per
 // point of any kind, in the order of memory, left whole warps and at last
 // one block waiting for a corner's 4096 dependent loads: 2.58 ms on
-// 48 x 44 x 40 x 36 against 0.067 ms here.
+// 48 x 44 x 40 x 36 against 0.054 ms here (0.067 before the point's coordinates
+// were taken apart in 32 bits and the loads of the sums and copies ran ahead);
+// a corner's chain alone is 0.031 (10^4).
 constexpr int kHaloThreads = 256;
 
 struct HaloParts {
@@ -146,52 +150,65 @@ __device__ double halo_weight(int m, int idx, double alpha) {
 }
 
 __global__ void __launch_bounds__(kHaloThreads) k_mpi_halo(double *__restrict__ f, HGrid h, HaloParts P) {
-  __shared__ double prod[4096];
+  __shared__ __align__(16) double prod[4096];
   int part = 0;
   while (part + 1 < P.parts && (int)blockIdx.x >= P.first[part + 1]) ++part;
   const int mask = P.mask[part];
-  const int blk = blockIdx.x - P.first[part];
+  const unsigned blk = blockIdx.x - P.first[part];
   if (mask == 0) {
     // Periodic images: one block per (vx, vy) of [-2, n + 1]; where both are
     // grid coordinates, only the two points around the (x, y) plane.
-    const int cvx = blk % (h.n[2] + 4) - 2, cvy = blk / (h.n[2] + 4) - 2;
+    const int cvx = (int)(blk % (h.n[2] + 4)) - 2, cvy = (int)(blk / (h.n[2] + 4)) - 2;
     const bool vin = cvx >= 0 && cvx < h.n[2] && cvy >= 0 && cvy < h.n[3];
     const int m0 = h.n[0] + 4, m1 = h.n[1] + 4;
     const int full = vin ? 4 * m0 : m0 * m1;
     const int count = vin ? full + 4 * h.n[1] : full;
-    const double *src = f + h.at(0, 0, wrapi(cvx, h.n[2]), wrapi(cvy, h.n[3]));
+    const double *src = f + h.at(0, 0, wrap1(cvx, h.n[2]), wrap1(cvy, h.n[3]));
     double *dst = f + h.at(0, 0, cvx, cvy);
-    for (int t = threadIdx.x; t < count; t += kHaloThreads) {
-      int cx, cy;
-      if (t < full) {  // whole rows
-        const int r = t / m0;
-        cx = t - r * m0 - 2;
-        cy = !vin || r < 2 ? r - 2 : h.n[1] + r - 2;
-      } else {  // two columns on each side of the grid's rows
-        const int k = (t - full) & 3;
-        cy = (t - full) >> 2;
-        cx = k < 2 ? k - 2 : h.n[0] + k - 2;
+    // Four points of a thread at a time, their loads ahead of their stores.
+    for (int t0 = threadIdx.x; t0 < count; t0 += 4 * kHaloThreads) {
+      double v[4];
+      int to[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int t = t0 + j * kHaloThreads;
+        if (t >= count) break;
+        int cx, cy;
+        if (t < full) {  // whole rows
+          const int r = t / m0;
+          cx = t - r * m0 - 2;
+          cy = !vin || r < 2 ? r - 2 : h.n[1] + r - 2;
+        } else {  // two columns on each side of the grid's rows
+          const int k = (t - full) & 3;
+          cy = (t - full) >> 2;
+          cx = k < 2 ? k - 2 : h.n[0] + k - 2;
+        }
+        to[j] = cx + h.is[1] * cy;
+        v[j] = src[wrap1(cx, h.n[0]) + h.is[1] * wrap1(cy, h.n[1])];
       }
-      dst[cx + h.s[1] * cy] = src[wrapi(cx, h.n[0]) + h.s[1] * wrapi(cy, h.n[1])];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (t0 + j * kHaloThreads < count) dst[to[j]] = v[j];
     }
     return;
   }
   const int m = __popc(mask);
   // Point index: a block, a warp or a thread each.
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int idx = m == 4 ? blk : (m == 3 ? blk * (kHaloThreads / 32) + warp : blk * kHaloThreads + (int)threadIdx.x);
-  long long total = 1LL << m, i = idx;
+  const unsigned idx = m == 4 ? blk : (m == 3 ? blk * (kHaloThreads / 32) + warp : blk * kHaloThreads + threadIdx.x);
+  unsigned total = 1u << m, i = idx;  // 2^32 points of one kind would be an array of 270 GB
   int c[4], st[4] = {0, 0, 0, 0};
   long long base = 0;  // of the sums: their terms are at base + sum_l st[l] j_l
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     c[k] = 0;
     if (!((mask >> k) & 1)) {
-      const int ext = h.n[k] + 4;
-      c[k] = (int)(i % ext) - 2;
-      i /= ext;
+      const unsigned ext = (unsigned)h.n[k] + 4;
+      const unsigned q = i / ext;
+      c[k] = (int)(i - q * ext) - 2;
+      i = q;
       total *= ext;
-      base += h.s[k] * (wrapi(c[k], h.n[k]) + kH);
+      base += h.s[k] * (wrap1(c[k], h.n[k]) + kH);
     }
   }
   int l = 0;
@@ -200,7 +217,7 @@ __global__ void __launch_bounds__(kHaloThreads) k_mpi_halo(double *__restrict__ 
     if ((mask >> k) & 1) {
       const int sg = (i >> l) & 1 ? 1 : -1;
       c[k] = sg < 0 ? -kH : h.n[k] + kH - 1;
-      base += h.s[k] * (wrapi(c[k] - sg, h.n[k]) + kH);
+      base += h.s[k] * (wrap1(c[k] - sg, h.n[k]) + kH);
       const int step = sg * h.is[k];
       if (l == 0) st[0] = step;
       else if (l == 1) st[1] = step;
@@ -226,8 +243,22 @@ __global__ void __launch_bounds__(kHaloThreads) k_mpi_halo(double *__restrict__ 
     if (m == 4) __syncthreads();
     else __syncwarp();
     if (me != 0 || !on) return;
-#pragma unroll 16
-    for (int t = 0; t < terms; ++t) sum = add(sum, pr[t]);
+    // The next sixteen products are on their way while sixteen are added.
+    const double2 *q = (const double2 *)pr;
+    double2 a[8], b[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a[k] = q[k];
+    for (int t = 0; t < terms; t += 32) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) b[k] = q[t / 2 + 8 + k];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum = add(add(sum, a[k].x), a[k].y);
+      const int n = t + 32 < terms ? t / 2 + 16 : 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) a[k] = q[n + k];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum = add(add(sum, b[k].x), b[k].y);
+    }
   } else if (m == 2) {
     if (!on) return;
     double w1 = h.alpha;
