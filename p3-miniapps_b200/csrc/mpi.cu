@@ -414,8 +414,11 @@ namespace {
 // Lines of a plane in shared memory, extended and prefiltered in place: line
 // l (of `lines`) starts at pl + l * ls, position k of it (0 .. n + 5) is st * k
 // further; positions 3 .. n + 2 are given, all are written.  G lanes share a
-// line, S points each (G S >= n + 4).  Lines outside [flo, fhi] are extended
-// only.  aL = alpha^(n + 3).
+// line, S points each (G S >= n + 4).  The left boundary sum e0 enters the
+// causal pass at position 0, which the segments hold where G S > n + 4; where
+// they fill the line exactly (n = 36, 68, 100, 132, 268, 540) lane 0 starts at
+// position 1 and adds e0 there.  Lines outside [flo, fhi] are extended only.
+// aL = alpha^(n + 3).
 template <int S, int G, int ST>
 __device__ __noinline__ void plane_lines(double *pl, int st_, int ls, int n, int lines, int flo, int fhi, double beta,
                                          double sqrt3, double aL) {
@@ -448,6 +451,7 @@ __device__ __noinline__ void plane_lines(double *pl, int st_, int ls, int n, int
     double *q = p + k0 * st;
 #pragma unroll
     for (int j = 0; j < S; ++j) v[j] = k0 + j >= 0 ? q[j * st] : 0.;
+    if (g == 0 && k0 == 1) v[0] += e0;  // no lane holds position 0
     seg_causal<S>(v);
     // The lanes' last values, summed up with alpha^S per lane.
     double x = v[S - 1], A = alpha_pow(S);

@@ -115,3 +115,50 @@ def test_fused_step_long_lines(pkg, cuda, n):
         else:
             want = interior(rest.run_mpi(f0, 1)[0])
     assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+
+
+def _split_edges():
+    """Line lengths n around every split of n + 4 points into G segments of S:
+    one point short of it, exact, one beyond, and exact without the first
+    segment (the second one then starts at the line's first point)."""
+    out = set()
+    for S, G in ((5, 8), (9, 8), (13, 8), (17, 8), (17, 16), (17, 32)):
+        out |= {S * G - 5, S * G - 4, S * G - 3, S * (G - 1) - 4}
+    return sorted(out)
+
+
+# (The fused step takes up to 512 points along x.)
+@pytest.mark.parametrize("dim,n", [(d, n) for d in range(4) for n in _split_edges() if d or n <= 512])
+def test_fused_step_split_edges(pkg, cuda, dim, n):
+    """The prefilter's lines at the edges of their splits into segments, along
+    each dimension, against the restated reference (the reference-order entry
+    points beyond its 512 points)."""
+    torch = cuda
+    size = [10, 11, 10, 12]
+    size[dim] = n
+    Lx, Ly = (L * max(1.0, size[d] / 60) for d in (0, 1))
+    rest = MpiRestatement(tuple(size), (0, 0, -VMAX, -VMAX), (Lx, Ly, VMAX, VMAX), DT, 10)
+    f0 = rest.init_halo(IC_SLD10)
+    # No symmetry about the box's ends: the boundary sums of both differ.
+    x, y = (np.arange(size[d] + 6) - 3 for d in (0, 1))
+    f0 *= (1 + 0.3 * np.sin(2 * np.pi * x / size[0] + 0.7))[None, None, None, :]
+    f0 *= (1 + 0.2 * np.sin(2 * np.pi * y / size[1] - 0.4))[None, None, :, None]
+    dom = pkg.Domain(size, [0.0, 0.0, -VMAX, -VMAX], [Lx, Ly, VMAX, VMAX], DT, 2, 10)
+    with pkg.Context(dom, "f64") as ctx:
+        out = ctx.mpi_run(torch.from_numpy(f0).cuda(), ctx.mpi_empty(), 1)
+        ctx.check()
+        got = interior(out.cpu().numpy())
+        if n + 6 > 512:
+            half, tmp = torch.from_numpy(f0).cuda(), ctx.mpi_empty()
+            ctx.mpi_halo_fill(half)
+            ctx.mpi_spline_xy(half)
+            new = half.clone()
+            ctx.mpi_advect_2d(half, tmp, 0.5 * DT)
+            ctx.mpi_field(half)
+            ctx.mpi_spline_vxvy(new)
+            ctx.mpi_advect_4d(new, tmp, DT)
+            ctx.check()
+            want = interior(new.cpu().numpy())
+        else:
+            want = interior(rest.run_mpi(f0, 1)[0])
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
