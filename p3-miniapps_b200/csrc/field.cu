@@ -354,7 +354,6 @@ int diags_async(vlp4d_ctx *c, int iter, cudaStream_t s) {
 
 int diags_join(vlp4d_ctx *c, cudaStream_t s) {
   VLP4D_CUDA_TRY(cudaStreamWaitEvent(s, c->ev_join, 0));
-  c->after_event = true;
   return VLP4D_OK;
 }
 

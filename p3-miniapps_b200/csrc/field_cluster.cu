@@ -517,8 +517,6 @@ int launch_field_transpose_cluster(vlp4d_ctx *c, const double *gex, const double
   a.norm = 1.0 / ((double)nx * ny);
   cudaLaunchAttribute attr[2] = {};
   cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, attr, s);
-  if (c->after_event) cfg.numAttrs = 1;  // see launch_dep
-  c->after_event = false;
   cfg.dynamicSmemBytes = field_t_bytes(nx, ny, c->field_cluster);
   const bool p2 = pow2_plane(nx, ny);
   if (c->field_cluster == 16)
@@ -541,8 +539,6 @@ int launch_field_cluster(vlp4d_ctx *c, double offset, cudaStream_t s) {
   a.normcoeff = 1.0 / (double)(nx * ny);
   cudaLaunchAttribute attr[2] = {};
   cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, attr, s);
-  if (c->after_event) cfg.numAttrs = 1;  // see launch_dep
-  c->after_event = false;
   const bool p2 = pow2_plane(nx, ny);
   if (c->field_cluster == 16)
     VLP4D_CUDA_TRY(cudaLaunchKernelEx(&cfg, p2 ? k_field_cluster<16, true> : k_field_cluster<16, false>, a));
