@@ -383,10 +383,10 @@ int vlp4d_ensemble_set_idle_limit(vlp4d_ensemble *ens, long long cycles);
  * n[d] + 6 in every dimension, first index -3 (HALO_PTS = 3, Config.hpp:7),
  * layout_left, vlp4d_mpi_size() elements, 16-byte aligned.  The context must
  * be FP64 with every grid dimension at least 10 (MMAX + 2, Init.cpp:85-89).
- * A foot outside the interpolation range sets the context's error word:
- * vlp4d_check then returns VLP4D_ERR_RANGE (the reference exits with "Time
- * step is too large", thrust/Advection.hpp:21-26).  All calls are
- * asynchronous on `stream`. */
+ * A foot outside the interpolation range, or one that is not a number, sets
+ * the context's error word and its point receives 0: vlp4d_check then returns
+ * VLP4D_ERR_RANGE (the reference exits with "Time step is too large",
+ * thrust/Advection.hpp:21-26).  All calls are asynchronous on `stream`. */
 size_t vlp4d_mpi_size(const vlp4d_ctx *ctx);
 /* initcase of vlp4d_mpi (miniapps/vlp4d_mpi/openmp/Init.cpp:126-277) for the
  * domain's idcase: 10 SLD10, 20 TSI20 (vlp4d_mpi's own formula), 2/5 CYL02/

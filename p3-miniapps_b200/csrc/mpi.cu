@@ -855,6 +855,11 @@ __device__ __forceinline__ void lag3w(double p, double c[3]) {
   }
 }
 
+// Whether coordinate x of a foot lies in dimension j's admissible range.  A NaN
+// (of dt, the field, or f through it) does not: a test for lying outside would
+// let it pass, and its cell index is INT_MIN.
+__device__ __forceinline__ bool in_range(const HGrid &h, double x, int j) { return x >= h.lo[j] && x <= h.hi[j]; }
+
 // computeFeet (thrust Advection.hpp:260-309): half-step predictor with the
 // cell's own field, the field interpolated (periodic 3x3 Lagrange) at the
 // predicted (x, y), then the full-step foot; vx, vy clamped to the domain.
@@ -930,7 +935,7 @@ __device__ __forceinline__ bool foot4d(const HGrid &h, const double *__restrict_
   bool ok = true;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    ok &= !(xs[j] < h.lo[j] || xs[j] > h.hi[j]);
+    ok &= in_range(h, xs[j], j);
     g[j] = EXACT ? mul(h.inv_dx[j], sub(xs[j], h.minp[j])) : h.inv_dx[j] * (xs[j] - h.minp[j]);
   }
   return ok;
@@ -1245,7 +1250,7 @@ __global__ void __launch_bounds__(TileShape<EXACT>::threads, 1)
               ok[q] = true;
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                ok[q] &= !(xs[j] < h.lo[j] || xs[j] > h.hi[j]);
+                ok[q] &= in_range(h, xs[j], j);
                 g[q][j] = EXACT ? mul(h.inv_dx[j], sub(xs[j], h.minp[j])) : h.inv_dx[j] * (xs[j] - h.minp[j]);
               }
             }
