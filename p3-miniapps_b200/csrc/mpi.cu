@@ -798,13 +798,14 @@ namespace {
 // 4x4 spline interpolation of the coefficients in tmp at
 // (x - dt vx, y - dt vy).  A foot outside [xmin-1, xmax] (in cells) sets
 // bit 2 of *err and the point receives 0.
-// Block (32 x, 8 y) of (ix, iy), a thread takes the planes p = z, z + G, ...
-// (48 x 44 x 40 x 36: 37 us; one thread per cell with its index taken apart by
-// 64-bit divisions, 45 us.)
+// A block is a tile of W x and H y (W H of its threads), a thread takes the
+// planes p = z, z + G, ...  With the call's copy, one box: 48 x 44 x 40 x 36 46 us,
+// 10 x 92 x 112 x 23 43 (one thread per cell with its index taken apart by 64-bit
+// divisions 63 and 52; blocks of 32 x 8 points 52 and 81).
 __global__ void __launch_bounds__(256) k_mpi_advect_2d(const double *__restrict__ tmp, double *__restrict__ fn,
-                                                       HGrid h, double dt, int *__restrict__ err) {
-  const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y;
-  if (ix >= h.n[0] || iy >= h.n[1]) return;
+                                                       HGrid h, int W, int H, double dt, int *__restrict__ err) {
+  const int ty = threadIdx.x / W, ix = blockIdx.x * W + (threadIdx.x - ty * W), iy = blockIdx.y * H + ty;
+  if (ty >= H || ix >= h.n[0] || iy >= h.n[1]) return;
   const int planes = h.n[2] * h.n[3];
   const double x = add(h.minp[0], mul((double)ix, h.dx[0]));
   const double y = add(h.minp[1], mul((double)iy, h.dx[1]));
@@ -1972,12 +1973,17 @@ int vlp4d_mpi_advect_2d(vlp4d_ctx *ctx, void *fn, void *fn_tmp, double dt, void 
   const HGrid h = make_hgrid(ctx);
   cudaStream_t s = (cudaStream_t)stream;
   VLP4D_CUDA_TRY(cudaMemcpyAsync(fn_tmp, fn, sizeof(double) * (size_t)h.total(), cudaMemcpyDeviceToDevice, s));
-  const dim3 grid((unsigned)((h.n[0] + 31) / 32), (unsigned)((h.n[1] + 7) / 8));
-  long long G = ((long long)ctx->num_sms * 16 + (long long)grid.x * grid.y - 1) / ((long long)grid.x * grid.y);
-  const long long planes = (long long)h.n[2] * h.n[3];
+  // Equal tiles of at most 32 columns and 256 points (a fixed 32 x 8 leaves 22
+  // lanes of 32 idle at nx = 10).
+  const int nxt = (h.n[0] + 31) / 32, W = (h.n[0] + nxt - 1) / nxt;
+  const int nyt = (h.n[1] + 256 / W - 1) / (256 / W), H = (h.n[1] + nyt - 1) / nyt;
+  const int threads = (W * H + 31) / 32 * 32;
+  // Sixteen blocks of 256 threads per SM.
+  const long long tiles = (long long)nxt * nyt, planes = (long long)h.n[2] * h.n[3];
+  long long G = ((long long)ctx->num_sms * 16 * 256 + tiles * threads - 1) / (tiles * threads);
   if (G > planes) G = planes;
-  k_mpi_advect_2d<<<dim3(grid.x, grid.y, (unsigned)G), dim3(32, 8), 0, s>>>((const double *)fn_tmp, (double *)fn, h, dt,
-                                                                            ctx->d_err);
+  k_mpi_advect_2d<<<dim3((unsigned)nxt, (unsigned)nyt, (unsigned)G), threads, 0, s>>>(
+      (const double *)fn_tmp, (double *)fn, h, W, H, dt, ctx->d_err);
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }

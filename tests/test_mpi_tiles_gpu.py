@@ -162,3 +162,21 @@ def test_fused_step_split_edges(pkg, cuda, dim, n):
         else:
             want = interior(rest.run_mpi(f0, 1)[0])
     assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("n", [(10, 10, 10, 10), (10, 26, 10, 11), (32, 8 + 3, 10, 10), (33, 17, 11, 10), (65, 12, 10, 10),
+                               (16, 257, 10, 10), (11, 300, 10, 10)])
+def test_advect_2d_bit_identical(pkg, cuda, n):
+    """The 2D advection at the edges of its (x, y) tiles."""
+    torch = cuda
+    Lx, Ly = (L * max(1.0, n[d] / 60) for d in (0, 1))
+    rest = MpiRestatement(n, (0, 0, -VMAX, -VMAX), (Lx, Ly, VMAX, VMAX), DT, 10)
+    c4 = np.random.default_rng(sum(n)).standard_normal(rest.init_halo(IC_SLD10).shape)
+    want, err = rest.advect_2d(c4, 0.5 * DT)
+    assert not err
+    dom = pkg.Domain(list(n), [0.0, 0.0, -VMAX, -VMAX], [Lx, Ly, VMAX, VMAX], DT, 2, 10)
+    with pkg.Context(dom, "f64") as ctx:
+        c, tmp = torch.from_numpy(c4).cuda(), ctx.mpi_empty()
+        ctx.mpi_advect_2d(c, tmp, 0.5 * DT)
+        ctx.check()
+        assert np.array_equal(c.cpu().numpy(), want)
