@@ -88,6 +88,20 @@ HGrid make_hgrid(const vlp4d_ctx *c) {
   return h;
 }
 
+// Equal (x, y) tiles of at most 32 columns and 256 points, a thread per point (a
+// fixed 32 x 8 leaves 22 lanes of 32 idle at nx = 10).  `rows`: a warp per row
+// of 32 columns where that leaves less than a fifth of the lanes idle.
+struct PlaneTiles {
+  int W, H, nxt, nyt, threads;
+  PlaneTiles(const HGrid &h, bool rows) {
+    nxt = (h.n[0] + 31) / 32;
+    W = rows && 5 * h.n[0] >= 4 * 32 * nxt ? 32 : (h.n[0] + nxt - 1) / nxt;
+    nyt = (h.n[1] + 256 / W - 1) / (256 / W);
+    H = (h.n[1] + nyt - 1) / nyt;
+    threads = (W * H + 31) / 32 * 32;
+  }
+};
+
 __device__ __forceinline__ int wrapi(int i, int n) { return ((i % n) + n) % n; }
 // The same for i in [-n, 2 n).
 __device__ __forceinline__ int wrap1(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
@@ -798,10 +812,10 @@ namespace {
 // 4x4 spline interpolation of the coefficients in tmp at
 // (x - dt vx, y - dt vy).  A foot outside [xmin-1, xmax] (in cells) sets
 // bit 2 of *err and the point receives 0.
-// A block is a tile of W x and H y (W H of its threads), a thread takes the
-// planes p = z, z + G, ...  With the call's copy, one box: 48 x 44 x 40 x 36 46 us,
-// 10 x 92 x 112 x 23 43 (one thread per cell with its index taken apart by 64-bit
-// divisions 63 and 52; blocks of 32 x 8 points 52 and 81).
+// A block is a tile of W x and H y (PlaneTiles), a thread takes the planes p = z,
+// z + G, ...  With the call's copy, one box: 48 x 44 x 40 x 36 46 us, 10 x 92 x 112 x
+// 23 43 (one thread per cell with its index taken apart by 64-bit divisions 63 and
+// 52; blocks of 32 x 8 points 52 and 81).
 __global__ void __launch_bounds__(256) k_mpi_advect_2d(const double *__restrict__ tmp, double *__restrict__ fn,
                                                        HGrid h, int W, int H, double dt, int *__restrict__ err) {
   const int ty = threadIdx.x / W, ix = blockIdx.x * W + (threadIdx.x - ty * W), iy = blockIdx.y * H + ty;
@@ -980,19 +994,20 @@ __device__ __forceinline__ double interp4d(const HGrid &h, const double *__restr
   return f1;
 }
 
-// Advection::advect_4D at the grid points: block (32 x, 8 y) of (ix, iy),
-// blockIdx.z = plane group; a thread takes the planes p = z, z + G, ...
+// Advection::advect_4D at the grid points: a block is a tile of W x and H y
+// (PlaneTiles), blockIdx.z = plane group; a thread takes the planes p = z, z + G, ...
 // (p = ivx + nvx*ivy).  MOMENT also accumulates the velocity moment
 // (part[z][ix + nx*iy]) and, per block, the sum of squares of the new
 // values (l2[block] as a (sum, 0) pair) for the field and the L2 norm.
 template <bool EXACT, bool MOMENT>
 __global__ void __launch_bounds__(256) k_mpi_advect_4d(const double *__restrict__ c, double *__restrict__ fn,
                                                        const double *__restrict__ ex, const double *__restrict__ ey,
-                                                       HGrid h, double dt, double *__restrict__ part,
-                                                       double *__restrict__ l2, int *__restrict__ err) {
-  const int ix = blockIdx.x * 32 + threadIdx.x, iy = blockIdx.y * 8 + threadIdx.y;
+                                                       HGrid h, int W, int H, double dt,
+                                                       double *__restrict__ part, double *__restrict__ l2,
+                                                       int *__restrict__ err) {
+  const int ty = threadIdx.x / W, ix = blockIdx.x * W + (threadIdx.x - ty * W), iy = blockIdx.y * H + ty;
   const int G = gridDim.z;
-  const bool live = ix < h.n[0] && iy < h.n[1];
+  const bool live = ty < H && ix < h.n[0] && iy < h.n[1];
   const long long planes = (long long)h.n[2] * h.n[3];
   double acc = 0., sq = 0.;
   bool bad = false;
@@ -1018,14 +1033,14 @@ __global__ void __launch_bounds__(256) k_mpi_advect_4d(const double *__restrict_
     if (live) part[(long long)blockIdx.z * h.n[0] * h.n[1] + ix + (long long)h.n[0] * iy] = acc;
     // Block sum of sq in a fixed order.
     __shared__ double ws[8];
-    const int tid = threadIdx.y * 32 + threadIdx.x;
+    const int tid = threadIdx.x;
     double v = sq;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if ((tid & 31) == 0) ws[tid >> 5] = v;
     __syncthreads();
     if (tid == 0) {
       double s = 0.;
-      for (int w = 0; w < 8; ++w) s += ws[w];
+      for (int w = 0; w < (int)blockDim.x / 32; ++w) s += ws[w];
       const long long b = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
       l2[2 * b] = s;
       l2[2 * b + 1] = 0.;
@@ -1796,13 +1811,13 @@ int launch_xy_pass(vlp4d_ctx *c, const HGrid &h, const double *fn, double *cxy, 
 template <bool EXACT, bool MOMENT>
 int launch_advect_4d(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn, double dt, int *groups,
                      long long *blocks, cudaStream_t s) {
-  const dim3 block(32, 8);
-  const long long bx = (h.n[0] + 31) / 32, by = (h.n[1] + 7) / 8;
+  const PlaneTiles t(h, true);
+  const long long bx = t.nxt, by = t.nyt;
   const long long planes = (long long)h.n[2] * h.n[3];
   // One resident wave: every block walks the planes p = z, z + G, ... at the
   // same pace, so the blocks in flight read neighbouring (vx, vy) slabs.
   int per_sm = 0;
-  VLP4D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mpi_advect_4d<EXACT, MOMENT>, 256, 0));
+  VLP4D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mpi_advect_4d<EXACT, MOMENT>, t.threads, 0));
   long long G = ((long long)c->num_sms * (per_sm > 0 ? per_sm : 1)) / (bx * by);
   if (G < 1) G = 1;
   if (G > planes) G = planes;
@@ -1812,8 +1827,8 @@ int launch_advect_4d(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn,
     if (G < 1) return fail_msg(VLP4D_ERR_UNSUPPORTED, "mpi 4D advection: too many (x, y) blocks for the partials");
   }
   const dim3 grid((unsigned)bx, (unsigned)by, (unsigned)G);
-  k_mpi_advect_4d<EXACT, MOMENT><<<grid, block, 0, s>>>(c4, fn, c->ex, c->ey, h, dt, c->rho_part, c->mpi_part,
-                                                         c->d_err);
+  k_mpi_advect_4d<EXACT, MOMENT><<<grid, t.threads, 0, s>>>(c4, fn, c->ex, c->ey, h, t.W, t.H, dt, c->rho_part,
+                                                             c->mpi_part, c->d_err);
   VLP4D_LAUNCH_CHECK();
   if (groups) *groups = (int)G;
   if (blocks) *blocks = G * bx * by;
@@ -1877,6 +1892,31 @@ bool tile4_config(const vlp4d_ctx *c, const HGrid &h, int cells, int threads, bo
   return best > 0.;
 }
 
+// Whether the tiles beat one thread per cell in the reference's arithmetic.  The
+// tiles pay for idle rims, for the slabs that mixed first taps add and, in one
+// round, for the slowest tile; a thread per cell reads all 256 taps through L1.
+// Both times are estimates, in us on 148 SMs, fitted to 460 grids of 10 to 96
+// points a side in fields of four modes (11 and 12% off, rms): tiles Q + 0.5
+// steps of 4.8 + 0.66 per warp, a quarter (a tenth) more where a vx (vy) grid line
+// has no velocity and its feet lie on either side; threads 0.12 ns per cell of
+// whole rows, up to 0.21 in tiles of short rows.  Over those grids the choice
+// gains 1.20 against tiles everywhere and 1.28 against one thread per cell in
+// blocks of 32 x 8 everywhere.  Tiles / threads: 26 x 16 x 16 x 14 40 / 20, 16^4
+// 31 / 18; 48 x 44 x 40 x 36 336 / 520, 38 x 55 x 72 x 64 1330 / 2230.
+bool tile4_faster(const vlp4d_ctx *c, const HGrid &h, const Tile4 &T) {
+  auto still = [&](int d) {  // a grid line of no velocity
+    const double k = std::round(-h.minp[d] / h.dx[d]);
+    return k >= 0. && k < h.n[d] && std::fabs(h.minp[d] + k * h.dx[d]) < 1e-9 * h.dx[d];
+  };
+  const int rounds = (T.nitems + c->num_sms - 1) / c->num_sms, warps = (T.W * T.YG * T.V + 31) / 32;
+  const double tiles = 5.6 + (rounds == 1 ? 1. : 0.8 * rounds) * (T.Q + 0.52) * (4.8 + 0.66 * warps) *
+                                 (1. + (still(2) ? 0.24 : 0.) + (still(3) ? 0.1 : 0.));
+  const PlaneTiles p(h, true);
+  const double kcells = 1e-3 * p.nxt * p.nyt * p.threads * h.n[2] * h.n[3];
+  const double threads = 8.7 + kcells * (p.W == 32 ? 0.1215 : 0.206 - 0.092 * h.n[0] / (32. * p.nxt));
+  return tiles < threads;
+}
+
 template <bool EXACT, bool MOMENT, int PXC>
 int run_advect_4d_tile(vlp4d_ctx *c, const HGrid &h, const Tile4 &T, const double *c4, double *fn, double dt,
                        long long *blocks, cudaStream_t s) {
@@ -1898,6 +1938,8 @@ int launch_advect_4d_any(vlp4d_ctx *c, const HGrid &h, const double *c4, double 
                          long long *blocks, cudaStream_t s) {
   Tile4 T;
   if (!c->fused || !tile4_config(c, h, TileShape<EXACT>::cells, TileShape<EXACT>::threads, MOMENT, T))
+    return launch_advect_4d<EXACT, MOMENT>(c, h, c4, fn, dt, groups, blocks, s);
+  if (EXACT && !c->fused_only && !tile4_faster(c, h, T))
     return launch_advect_4d<EXACT, MOMENT>(c, h, c4, fn, dt, groups, blocks, s);
   if (groups) *groups = T.nvt * T.nseg;
   if (T.PX == 36) return run_advect_4d_tile<EXACT, MOMENT, 36>(c, h, T, c4, fn, dt, blocks, s);
@@ -1973,17 +2015,13 @@ int vlp4d_mpi_advect_2d(vlp4d_ctx *ctx, void *fn, void *fn_tmp, double dt, void 
   const HGrid h = make_hgrid(ctx);
   cudaStream_t s = (cudaStream_t)stream;
   VLP4D_CUDA_TRY(cudaMemcpyAsync(fn_tmp, fn, sizeof(double) * (size_t)h.total(), cudaMemcpyDeviceToDevice, s));
-  // Equal tiles of at most 32 columns and 256 points (a fixed 32 x 8 leaves 22
-  // lanes of 32 idle at nx = 10).
-  const int nxt = (h.n[0] + 31) / 32, W = (h.n[0] + nxt - 1) / nxt;
-  const int nyt = (h.n[1] + 256 / W - 1) / (256 / W), H = (h.n[1] + nyt - 1) / nyt;
-  const int threads = (W * H + 31) / 32 * 32;
+  const PlaneTiles t(h, false);
   // Sixteen blocks of 256 threads per SM.
-  const long long tiles = (long long)nxt * nyt, planes = (long long)h.n[2] * h.n[3];
-  long long G = ((long long)ctx->num_sms * 16 * 256 + tiles * threads - 1) / (tiles * threads);
+  const long long tiles = (long long)t.nxt * t.nyt, planes = (long long)h.n[2] * h.n[3];
+  long long G = ((long long)ctx->num_sms * 16 * 256 + tiles * t.threads - 1) / (tiles * t.threads);
   if (G > planes) G = planes;
-  k_mpi_advect_2d<<<dim3((unsigned)nxt, (unsigned)nyt, (unsigned)G), threads, 0, s>>>(
-      (const double *)fn_tmp, (double *)fn, h, W, H, dt, ctx->d_err);
+  k_mpi_advect_2d<<<dim3((unsigned)t.nxt, (unsigned)t.nyt, (unsigned)G), t.threads, 0, s>>>(
+      (const double *)fn_tmp, (double *)fn, h, t.W, t.H, dt, ctx->d_err);
   VLP4D_LAUNCH_CHECK();
   return VLP4D_OK;
 }

@@ -26,7 +26,7 @@ def _range_error(pkg, ctx):
     ctx.check()  # reported once
 
 
-@pytest.mark.parametrize("kernels", ["auto", "generic"])
+@pytest.mark.parametrize("kernels", ["auto", "fused", "generic"])
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 @pytest.mark.parametrize("n", SHAPES)
 def test_field_not_finite(pkg, cuda, monkeypatch, n, value, kernels):

@@ -180,3 +180,13 @@ def test_advect_2d_bit_identical(pkg, cuda, n):
         ctx.mpi_advect_2d(c, tmp, 0.5 * DT)
         ctx.check()
         assert np.array_equal(c.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("kernels", ["fused", "generic"])
+@pytest.mark.parametrize("cells", [0.4, 2.7])
+@pytest.mark.parametrize("n", SHAPES + [(28, 11, 10, 10), (26, 19, 10, 12), (45, 10, 12, 10)])
+def test_advect_4d_both_routes(pkg, cuda, monkeypatch, n, cells, kernels):
+    """The reference-order 4D advection by tiles and by one thread per cell,
+    whichever the size would choose."""
+    monkeypatch.setenv("VLP4D_KERNELS", kernels)
+    test_advect_4d_bit_identical(pkg, cuda, n, cells)
