@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include <string>
 
 #include "../../include/vlp4d_b200.h"
@@ -90,6 +91,23 @@ struct StencilTable {
   unsigned long long stamp = 0;  // last use, for slot replacement
 };
 
+// Geometry of the tiles of the vlp4d_mpi 4D advection (mpi.cu); vy in nseg
+// segments of Q.
+struct Tile4 {
+  int R, W, YG, V;       // cells of a thread, x extent, groups of R y, vx extent
+  int PX, RY, RV, slab;  // W + 4, R YG + 4, V + 4, PX * RY * RV
+  unsigned magic;        // ceil(2^32 / PX): i / PX for i < 2^16
+  int nxt, nyt, nvt, Q, nseg;
+  int nitems;
+};
+
+// The tiles of a context, and whether its size runs by them.
+struct MpiTiles {
+  std::once_flag once;
+  bool use = false;
+  Tile4 T;
+};
+
 }  // namespace vlp4d
 
 struct vlp4d_ctx {
@@ -166,6 +184,8 @@ struct vlp4d_ctx {
   // pass (mpi.cu), mpi_part_cap pairs.
   double *mpi_part = nullptr;
   int mpi_part_cap = 0;
+  // Tiles of the 4D pass of the fused step [0] and of the reference-order call [1].
+  vlp4d::MpiTiles mpi_tiles[2];
 
   // vy-slab contexts (vlp4d_ctx_create_slab): this context owns the global
   // vy planes [ivy0, ivy0 + g.n[3]) of a run with nvy_glob planes.  g holds

@@ -1057,14 +1057,7 @@ __global__ void __launch_bounds__(256) k_mpi_advect_4d(const double *__restrict_
 // read from shared memory once for all of them, 112 (160) loads per cell
 // instead of 256.
 //
-// Geometry of the tiles; vy in nseg segments of Q.
-struct Tile4 {
-  int R, W, YG, V;       // cells of a thread, x extent, groups of R y, vx extent
-  int PX, RY, RV, slab;  // W + 4, R YG + 4, V + 4, PX * RY * RV
-  unsigned magic;        // ceil(2^32 / PX): i / PX for i < 2^16
-  int nxt, nyt, nvt, Q, nseg;
-  int nitems;
-};
+// Tile4 (internal.cuh) is the geometry of the tiles.
 // Cells of a thread (consecutive in y) and threads of a block.  Measured, us,
 // four cells and 256 threads (255 registers) against two and 512 (128): fused
 // 128 x 128 x 64 x 64 4343 / 5052, 64^4 1271 / 1349, 48 x 44 x 40 x 36 331 / 338;
@@ -1936,11 +1929,14 @@ int run_advect_4d_tile(vlp4d_ctx *c, const HGrid &h, const Tile4 &T, const doubl
 template <bool EXACT, bool MOMENT>
 int launch_advect_4d_any(vlp4d_ctx *c, const HGrid &h, const double *c4, double *fn, double dt, int *groups,
                          long long *blocks, cudaStream_t s) {
-  Tile4 T;
-  if (!c->fused || !tile4_config(c, h, TileShape<EXACT>::cells, TileShape<EXACT>::threads, MOMENT, T))
-    return launch_advect_4d<EXACT, MOMENT>(c, h, c4, fn, dt, groups, blocks, s);
-  if (EXACT && !c->fused_only && !tile4_faster(c, h, T))
-    return launch_advect_4d<EXACT, MOMENT>(c, h, c4, fn, dt, groups, blocks, s);
+  // Sought once per context: up to 60 us of host time (10 x 10 x 100 x 300).
+  MpiTiles &tiles = c->mpi_tiles[EXACT];
+  std::call_once(tiles.once, [&] {
+    tiles.use = c->fused && tile4_config(c, h, TileShape<EXACT>::cells, TileShape<EXACT>::threads, MOMENT, tiles.T) &&
+                (!EXACT || c->fused_only || tile4_faster(c, h, tiles.T));
+  });
+  if (!tiles.use) return launch_advect_4d<EXACT, MOMENT>(c, h, c4, fn, dt, groups, blocks, s);
+  const Tile4 &T = tiles.T;
   if (groups) *groups = T.nvt * T.nseg;
   if (T.PX == 36) return run_advect_4d_tile<EXACT, MOMENT, 36>(c, h, T, c4, fn, dt, blocks, s);
   return run_advect_4d_tile<EXACT, MOMENT, 0>(c, h, T, c4, fn, dt, blocks, s);
