@@ -216,12 +216,12 @@ __global__ void __launch_bounds__(kVColsThreads, 4) k_v_cols(VCols a) {
   T wx[6], wy[6];
   int jx = ivx0, jy = iv0;
   if (DVX) {
-    load_weights_cg(WeightsOf<T>::get(a.tvx), col, wx);
-    jx += __ldcg(a.tvx.m + col);
+    load_weights_dep(WeightsOf<T>::get(a.tvx), col, wx);
+    jx += a.tvx.m[col];
   }
   if (DVY) {
-    load_weights_cg(WeightsOf<T>::get(a.tvy), col, wy);
-    jy = (iv0 + __ldcg(a.tvy.m + col)) % a.nvy;
+    load_weights_dep(WeightsOf<T>::get(a.tvy), col, wy);
+    jy = (iv0 + a.tvy.m[col]) % a.nvy;
   }
   int off[NT];
   jx %= a.nvx;

@@ -204,9 +204,9 @@ __global__ void __launch_bounds__(512) k_vslab(const __grid_constant__ CUtensorM
     {
       int j = vx0;
       if (DVX) {
-        j += __ldcg(a.tvx.m + ixy);
+        j += a.tvx.m[ixy];
         if (j >= nvx) j -= nvx;
-        load_weights_cg(WeightsOf<T>::get(a.tvx), ixy, wvx);
+        load_weights_dep(WeightsOf<T>::get(a.tvx), ixy, wvx);
       }
 #pragma unroll
       for (int q = 0; q < V + 5; ++q) {
@@ -215,11 +215,11 @@ __global__ void __launch_bounds__(512) k_vslab(const __grid_constant__ CUtensorM
       }
     }
     if (DVY) {
-      lag0 = 5 + signed_offset(__ldcg(a.tvy.m + ixy), a.nvy) - a.span[cc].x;
-      load_weights_cg(WeightsOf<T>::get(a.tvy), ixy, wvy);
+      lag0 = 5 + signed_offset(a.tvy.m[ixy], a.nvy) - a.span[cc].x;
+      load_weights_dep(WeightsOf<T>::get(a.tvy), ixy, wvy);
     }
     constexpr bool has_bias = BIAS;
-    const double bias = BIAS ? a.bias_scale * __ldcg(a.bias + ixy) : 0.0;
+    const double bias = BIAS ? a.bias_scale * a.bias[ixy] : 0.0;
     // Output pointer of the next row this thread writes.
     T *orow = static_cast<T *>(a.fout) + ixy + vstride * vx0 + ystride * (long long)sg * a.Q;
     // Ring of vx-swept rows, slot = t % 6 (static after unrolling).  FP64:

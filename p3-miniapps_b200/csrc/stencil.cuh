@@ -135,12 +135,16 @@ __device__ __forceinline__ void load_weights(const T *__restrict__ w, long long 
   for (int k = 0; k < 6; ++k) out[k] = __ldg(w + 6 * line + k);
 }
 
-// The same through L2, for tables that the kernel before may still be writing
-// when this one starts.
+// The same by plain loads, for tables that the kernel before may still be
+// writing when this one starts (after pdl_wait; the read-only path is closed to
+// them).  Not past L1: every thread row and segment reads its columns' weights
+// again, and on a plane of few columns all CTAs the same lines (us, through L2
+// against L1: v-slab pass of 8 x 4 x 128 x 128 FP64, an output row per item, vx 25.9 /
+// 6.9, both 34.9 / 14.9; column pass of 8 x 8 x 96 x 47 FP64, both 15.6 / 7.2).
 template <typename T>
-__device__ __forceinline__ void load_weights_cg(const T *w, long long line, T (&out)[6]) {
+__device__ __forceinline__ void load_weights_dep(const T *w, long long line, T (&out)[6]) {
 #pragma unroll
-  for (int k = 0; k < 6; ++k) out[k] = __ldcg(w + 6 * line + k);
+  for (int k = 0; k < 6; ++k) out[k] = w[6 * line + k];
 }
 
 }  // namespace vlp4d
