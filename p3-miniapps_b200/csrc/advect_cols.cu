@@ -359,9 +359,25 @@ int run_v_cols(vlp4d_ctx *c, VCols &a, cudaStream_t s) {
 
 }  // namespace
 
+// Narrow planes leave most lanes of a tile's loads and sweeps idle, and planes
+// of few cells most threads of a block: there one thread per output is faster
+// (us, columns against threads: x, 11 x 38 x 88 x 48 FP32 18.3 / 14.4 and 9 x 64 x 64
+// x 104 43.0 / 26.7; y, 11 x 38 x 88 x 48 22.7 / 14.4; x and y, 2 x 16 x 104 x 120 35.6 / 10.3
+// and 1 x 87 x 48 x 62 34.5 / 8.2; with the moment 31.2 / 16.4).  The lines lie where
+// the two are equal over 700 grids of 1 to 70 columns; a pair's 36 loads per output,
+// and its moment as a pass of its own, make up for more idle lanes.
+bool xy_cols_pay(const vlp4d_ctx *c, bool x, bool y, bool with_rho) {
+  const int nx = c->g.n[0], ny = c->g.n[1];
+  const long long nxy = c->g.nxy();
+  if (x && y) return with_rho ? nx >= 4 && nxy >= 64 : nx >= 8 && ny >= 4 && nxy >= 64;
+  return x ? nx >= (c->dtype == VLP4D_F32 ? 20 : 24) && nxy >= 128 : nx >= 17 && nxy >= 256;
+}
+
 int launch_xy_cols(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTable *tx, const StencilTable *ty, int taps,
                    bool with_rho, cudaStream_t s) {
-  if (!c->fused || (!tx && !ty) || (taps == 11 && !(tx && ty)) || (with_rho && !(tx && ty))) return VLP4D_ERR_UNSUPPORTED;
+  if (!c->fused || (!tx && !ty) || (taps == 11 && !(tx && ty)) || (with_rho && !(tx && ty)) ||
+      !xy_cols_pay(c, tx, ty, with_rho))
+    return VLP4D_ERR_UNSUPPORTED;
   XyCols a;
   a.fin = fn;
   a.fout = fnp1;

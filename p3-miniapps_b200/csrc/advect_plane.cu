@@ -1495,7 +1495,7 @@ int launch_advect_xy(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTabl
   // per thread outside the in-place form (72 x 60 in chunks of 30: 168 / 155 us,
   // 80 x 90 in 18: 242 / 154; four rows per thread, 100 x 100 in 20: 82 / 104).
   // Both are left only where overlap_rows finds nothing.
-  if (!c->fused_only && do_x && do_y &&
+  if (!c->fused_only && do_x && do_y && xy_cols_pay(c, true, true, with_rho) &&
       (cfg.R < 5 && cfg.R < c->g.n[1] || (c->elem == 8 && !cfg.inplace && cfg.rt == 1)))
     return VLP4D_ERR_UNSUPPORTED;
   const bool moment = with_rho && do_x && do_y;

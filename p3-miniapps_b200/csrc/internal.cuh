@@ -321,7 +321,9 @@ int launch_advect_xyxy_tables(vlp4d_ctx *c, const void *fn, void *fnp1, const St
 // advect_cols.cu: x/y (6-tap lines, or the composed 11-tap ones with taps =
 // 11; the moment of the result into rho when with_rho) and vx/vy sweeps of
 // any shape and alignment.  VLP4D_ERR_UNSUPPORTED (nothing launched) under
-// VLP4D_KERNELS=generic and for index ranges beyond 32 bits.
+// VLP4D_KERNELS=generic, for index ranges beyond 32 bits and where one thread
+// per output is faster (xy_cols_pay).
+bool xy_cols_pay(const vlp4d_ctx *c, bool x, bool y, bool with_rho);
 int launch_xy_cols(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTable *tx, const StencilTable *ty, int taps,
                    bool with_rho, cudaStream_t s);
 int launch_v_cols(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTable *tvx, const StencilTable *tvy,

@@ -116,3 +116,12 @@ def test_overlapping_row_chunks(pkg, cuda, monkeypatch, n, dtype):
         fz.advect_xy_moment(half, want, 0.21)
         fz.check()
         assert float((out - want).abs().max()) <= (1e-13 if dtype == "f64" else 2e-6) * float(want.abs().max())
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("n", [(24, 6, 7, 5), (24, 5, 7, 5), (23, 6, 5, 7), (20, 13, 5, 7), (20, 12, 9, 4), (19, 14, 3, 8), (8, 12, 9, 7),
+                               (8, 11, 7, 9), (7, 14, 6, 8), (26, 4, 6, 5), (34, 3, 6, 5), (4, 16, 9, 7), (5, 13, 9, 7), (5, 12, 9, 7),
+                               (3, 22, 6, 9), (19, 5, 9, 8), (16, 6, 9, 8), (127, 1, 9, 8), (128, 1, 8, 9), (1, 129, 9, 8)])
+def test_routes_on_either_side(pkg, cuda, monkeypatch, n, dtype):
+    """Planes just inside and just outside of what the column kernels take."""
+    test_same_bits_as_cell_per_thread(pkg, cuda, monkeypatch, n, dtype)
