@@ -246,6 +246,14 @@ struct VgPair<double> {
   static __device__ __forceinline__ P fma2(P a, P b, P c) { return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)); }
 };
 
+// Bytes of k_vgrad_v's ring for nth threads, up to a multiple of 8 for the sums
+// that follow (13 floats and three rows of an odd number of threads, nvx = 116 or
+// 132, are not).
+template <typename T, int V, int S>
+__host__ __device__ constexpr size_t vgrad_ring(int nth) {
+  return (sizeof(T) * S * (2 * V + 5) * (size_t)nth + 7) / 8 * 8;
+}
+
 // The same sums with the vx taps shared: thread (cw, g) of a block owns
 // column ixy = blockIdx.x*CW + cw and the V consecutive output vx rows
 // g*V .. g*V+V-1 (blockDim = CW x nvx/V), so one input row costs V+5 loads
@@ -274,7 +282,7 @@ __global__ void __launch_bounds__(512) k_vgrad_v(const T *__restrict__ a, const 
   const int cw = threadIdx.x, g = threadIdx.y;
   const int nth = CW * G, tid = g * CW + cw;
   T *ring = reinterpret_cast<T *>(vg_smem);                               // [S][nth][NE]
-  double *red = reinterpret_cast<double *>(vg_smem + sizeof(T) * S * NE * nth);  // [2][G][CW]
+  double *red = reinterpret_cast<double *>(vg_smem + vgrad_ring<T, V, S>(nth));  // [2][G][CW]
   const int ixy = blockIdx.x * CW + cw;
   const int seg = blockIdx.y;
   const int ivy0 = seg * Q;
@@ -409,7 +417,7 @@ constexpr int vgrad_slots() {
 }
 template <typename T, int V>
 size_t vgrad_smem(int nth, int gy, int cw) {
-  return sizeof(T) * vgrad_slots<T, V>() * (2 * V + 5) * (size_t)nth + sizeof(double) * 2 * gy * cw;
+  return vgrad_ring<T, V, vgrad_slots<T, V>()>(nth) + sizeof(double) * 2 * gy * cw;
 }
 
 __global__ void k_vgrad_finish(const double *__restrict__ part, int nseg, int nxy, double *__restrict__ gex,
