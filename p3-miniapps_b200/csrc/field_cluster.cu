@@ -26,8 +26,10 @@
 //   -- cluster barrier (no CTA leaves while another reads its memory) --
 // Lines of power-of-two length use radix-4 Stockham passes (self-sorting,
 // one CTA barrier per pass over all lines of a phase; a radix-2 pass last
-// for odd powers); other lengths two sums of their largest factors (a prime
-// one direct sum).  Twiddles exp(2 pi i m / n) from sincospi.  All waits are the
+// for odd powers); other lengths two sums of their largest factors (short and
+// prime ones one direct sum).  Against the solve in extended precision (rms over
+// the plane, 15 planes of 9 to 72 points a side) their error is 0.97 of cuFFT's
+// with the mean of the density taken out and 0.49 with it left in.  All waits are the
 // hardware's CTA and cluster barriers, which every thread of every CTA
 // reaches the same number of times.
 #include <cstdlib>
@@ -69,6 +71,60 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
+// exp(2 pi i m / n).  Where n is no power of two the angle is reduced to the first
+// octant in whole numbers: 2 m / n itself is rounded by up to a unit of 2, seven
+// times the rounding of the sine.
+template <bool POW2>
+__device__ __forceinline__ double2 twiddle(int m, int n) {
+  double sn, cs;
+  if (POW2) {
+    sincospi(2.0 * m / n, &sn, &cs);
+    return make_double2(cs, sn);
+  }
+  const int o = 8 * m / n, r = 8 * m - o * n;  // octant, remainder of n
+  sincospi((double)(o & 1 ? n - r : r) / (4 * n), &sn, &cs);
+  const bool swap = ((o + 1) >> 1) & 1;  // octants 1, 2, 5, 6
+  const double re = swap ? sn : cs, im = swap ? cs : sn;
+  return make_double2(o >= 2 && o < 6 ? -re : re, o >= 4 ? -im : im);
+}
+
+// sum over j < N of x[j stride] w^(j step), w = exp(+-2 pi i / n), N step a
+// multiple of n.  Where step is not 0 the powers of w add up to 0: with `rel` the
+// terms are taken relative to the mean of four of them, so that the rounding of
+// the twiddles does not show at the scale of a density's mean beside its
+// perturbation.  Two chains of fused products, the loop not unrolled: a solve runs
+// from a cold instruction cache (four chains unrolled: 12 us more per solve in the
+// loop of 72 x 60 x 96 x 80).
+__device__ __forceinline__ double2 dft_sum(const double2 *x, int stride, int N, const double2 *tw, int step, int n,
+                                           bool inverse, bool rel) {
+  const double sgn = inverse ? 1. : -1.;
+  const double2 v0 = x[0];
+  double2 x0 = make_double2(0., 0.);
+  if (rel) {
+    const double2 a = x[N / 4 * stride], b = x[N / 2 * stride], c = x[3 * N / 4 * stride];
+    x0 = make_double2(0.25 * ((v0.x + a.x) + (b.x + c.x)), 0.25 * ((v0.y + a.y) + (b.y + c.y)));
+  }
+  double re[2] = {v0.x - x0.x, 0.}, im[2] = {v0.y - x0.y, 0.};
+  int m = 0;
+  auto term = [&](int j, int q) {
+    m += step;
+    if (m >= n) m -= n;
+    const double2 v = x[j * stride], t = tw[m];
+    const double dx = v.x - x0.x, dy = v.y - x0.y, wi = sgn * t.y;
+    re[q] = fma(dx, t.x, fma(-dy, wi, re[q]));
+    im[q] = fma(dx, wi, fma(dy, t.x, im[q]));
+  };
+  int j = 1;
+#pragma unroll 1
+  for (; j + 2 <= N; j += 2) {
+    term(j, 0);
+    term(j + 1, 1);
+  }
+  if (j < N) term(j, 0);
+  const double back = step == 0 ? N : 0;
+  return make_double2(fma(back, x0.x, re[0] + re[1]), fma(back, x0.y, im[0] + im[1]));
+}
+
 // DFT of `lines` contiguous lines of length n (line l at buf + l * n):
 // out[k] = sum_j in[j] w^(jk), w = exp(sign 2 pi i / n), tw[m] = exp(2 pi i
 // m / n) (conjugated for sign < 0).  The result is in buf or tmp (returned);
@@ -76,7 +132,8 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 // POW2: both lengths of the plane are powers of two, and the general code is
 // not compiled in (with it the 64 x 64 solve took 11.6 us instead of 9.9).
 template <bool POW2>
-__device__ double2 *line_dft(double2 *buf, double2 *tmp, int lines, int n, const double2 *tw, bool inverse) {
+__device__ double2 *line_dft(double2 *buf, double2 *tmp, int lines, int n, const double2 *tw, bool inverse,
+                             bool rel = false) {
   const double sgn = inverse ? 1. : -1.;
   if (POW2 || (n & (n - 1)) == 0) {
     const int ln = __ffs(n) - 1;  // log2(n)
@@ -137,28 +194,20 @@ __device__ double2 *line_dft(double2 *buf, double2 *tmp, int lines, int n, const
     return x;
   }
   // Other lengths, n = n1 n2 (n1 = 1 for primes): j = j1 n2 + j2, k = k1 + n1
-  // k2; sums over j1, a twiddle, sums over j2: n1 + n2 terms per value.
-  const int n1 = dft_factor(n), n2 = n / n1;
+  // k2; sums over j1, a twiddle, sums over j2: n1 + n2 terms per value.  Up to
+  // 32 points one sum of n terms: a second pass and its barrier cost more (us per
+  // solve in a graph, two sums / one: 9 x 16 7.4 / 6.1, 20 x 20 9.3 / 8.0, 24 x 24 9.5 /
+  // 8.8; with the bound at 48, 45 x 39 12.2 / 13.8).
+  const int n1 = n <= 32 ? 1 : dft_factor(n), n2 = n / n1;
   const double2 *x = buf;
   double2 *y = tmp;
   if (n1 > 1) {
     for (int o = threadIdx.x; o < lines * n; o += blockDim.x) {
       const int l = o / n, q = o - l * n;
       const int k1 = q / n2, j2 = q - k1 * n2;
-      const double2 *xl = buf + (size_t)l * n + j2;
-      const int step = k1 * n2;  // below n
-      double sr = 0., si = 0.;
-      int m = 0;
-      for (int j1 = 0; j1 < n1; ++j1) {
-        const double2 v = xl[j1 * n2], t = tw[m];
-        const double wi = sgn * t.y;
-        sr += v.x * t.x - v.y * wi;
-        si += v.x * wi + v.y * t.x;
-        m += step;
-        if (m >= n) m -= n;
-      }
+      const double2 s = dft_sum(buf + (size_t)l * n + j2, n2, n1, tw, k1 * n2, n, inverse, rel);
       const double2 t = tw[j2 * k1];  // below n
-      tmp[o] = cmul(make_double2(sr, si), make_double2(t.x, sgn * t.y));
+      tmp[o] = cmul(s, make_double2(t.x, sgn * t.y));
     }
     __syncthreads();
     x = tmp;
@@ -167,19 +216,7 @@ __device__ double2 *line_dft(double2 *buf, double2 *tmp, int lines, int n, const
   for (int o = threadIdx.x; o < lines * n; o += blockDim.x) {
     const int l = o / n, k = o - l * n;
     const int k2 = k / n1, k1 = k - k2 * n1;
-    const double2 *xl = x + (size_t)l * n + k1 * n2;
-    const int step = k2 * n1;  // below n
-    double sr = 0., si = 0.;
-    int m = 0;
-    for (int j2 = 0; j2 < n2; ++j2) {
-      const double2 v = xl[j2], t = tw[m];
-      const double wi = sgn * t.y;
-      sr += v.x * t.x - v.y * wi;
-      si += v.x * wi + v.y * t.x;
-      m += step;
-      if (m >= n) m -= n;
-    }
-    y[o] = make_double2(sr, si);
+    y[o] = dft_sum(x + (size_t)l * n + k1 * n2, 1, n2, tw, k2 * n1, n, inverse, rel);
   }
   __syncthreads();
   return y;
@@ -226,24 +263,22 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster(FieldArgs a) {
   double2 *twy = twx + nx;
   const unsigned c = cluster_rank();
   for (int m = threadIdx.x; m < nx; m += blockDim.x) {
-    double sn, cs;
-    sincospi(2.0 * m / nx, &sn, &cs);
-    twx[m] = make_double2(cs, sn);
+    twx[m] = twiddle<POW2>(m, nx);
   }
   for (int m = threadIdx.x; m < ny; m += blockDim.x) {
-    double sn, cs;
-    sincospi(2.0 * m / ny, &sn, &cs);
-    twy[m] = make_double2(cs, sn);
+    twy[m] = twiddle<POW2>(m, ny);
   }
   pdl_wait();
   pdl_trigger();
+  // A density whose mean the caller leaves in (idcase 110).
+  const bool rel = a.offset == 0.;
   // 1. Own rows along x (the last CTAs may have fewer than R, or none).
   const int iy0 = (int)c * R;
   const int nr = ny - iy0 < R ? (ny - iy0 > 0 ? ny - iy0 : 0) : R;
   for (int i = threadIdx.x; i < nr * nx; i += blockDim.x)
     rowA[i] = make_double2(a.rho[(size_t)iy0 * nx + i] - a.offset, 0.);
   __syncthreads();
-  const double2 *rows = line_dft<POW2>(rowA, rowB, nr, nx, twx, false);
+  const double2 *rows = line_dft<POW2>(rowA, rowB, nr, nx, twx, false, rel);
   cluster_barrier();
   // 2. Own columns along y: column q is kx = c + q * C (Kc slots; the last
   // ones of some CTAs are past nx/2 and stay unused).
@@ -255,7 +290,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster(FieldArgs a) {
     colA[i] = ld_cluster(rows + (size_t)(iy % R) * nx + kx, (unsigned)(iy / R));
   }
   __syncthreads();
-  const double2 *rhat = line_dft<POW2>(colA, colB, nq, ny, twy, false);
+  const double2 *rhat = line_dft<POW2>(colA, colB, nq, ny, twy, false, rel);
   // 3. The mode-wise solve into the other column buffer: spectra
   // phi_hat, ex_hat, ey_hat at slots [0, Kc), [Kc, 2Kc), [2Kc, 3Kc).
   double2 *spec = rhat == colA ? colB : colA;
@@ -340,14 +375,10 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster_t(FieldTArgs a)
   double2 *twy = twx + nx;
   const unsigned c = cluster_rank();
   for (int m = threadIdx.x; m < nx; m += blockDim.x) {
-    double sn, cs;
-    sincospi(2.0 * m / nx, &sn, &cs);
-    twx[m] = make_double2(cs, sn);
+    twx[m] = twiddle<POW2>(m, nx);
   }
   for (int m = threadIdx.x; m < ny; m += blockDim.x) {
-    double sn, cs;
-    sincospi(2.0 * m / ny, &sn, &cs);
-    twy[m] = make_double2(cs, sn);
+    twy[m] = twiddle<POW2>(m, ny);
   }
   pdl_wait();
   pdl_trigger();
