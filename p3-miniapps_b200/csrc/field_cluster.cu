@@ -356,7 +356,7 @@ __host__ __device__ inline size_t field_t_bytes(int nx, int ny, int ctas) {
   return sizeof(double2) * (4 * L.rows_elems + 4 * (size_t)L.Kc * ny + nx + ny);
 }
 
-template <int kFieldCtas, bool POW2>
+template <int kFieldCtas>
 __global__ void __launch_bounds__(kFieldThreads) k_field_cluster_t(FieldTArgs a) {
   extern __shared__ __align__(16) unsigned char fsm[];
   const int nx = a.nx, ny = a.ny, nxh = nx / 2 + 1;
@@ -375,10 +375,10 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster_t(FieldTArgs a)
   double2 *twy = twx + nx;
   const unsigned c = cluster_rank();
   for (int m = threadIdx.x; m < nx; m += blockDim.x) {
-    twx[m] = twiddle<POW2>(m, nx);
+    twx[m] = twiddle<true>(m, nx);
   }
   for (int m = threadIdx.x; m < ny; m += blockDim.x) {
-    twy[m] = twiddle<POW2>(m, ny);
+    twy[m] = twiddle<true>(m, ny);
   }
   pdl_wait();
   pdl_trigger();
@@ -389,8 +389,8 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster_t(FieldTArgs a)
     ry[i] = make_double2(a.gey[(size_t)iy0 * nx + i], 0.);
   }
   __syncthreads();
-  const double2 *rowsx = line_dft<POW2>(rx, rxt, nr, nx, twx, false);
-  const double2 *rowsy = line_dft<POW2>(ry, ryt, nr, nx, twx, false);
+  const double2 *rowsx = line_dft<true>(rx, rxt, nr, nx, twx, false);
+  const double2 *rowsy = line_dft<true>(ry, ryt, nr, nx, twx, false);
   cluster_barrier();
   int nq = 0;
   for (int kx = (int)c; kx < nxh; kx += kFieldCtas) ++nq;
@@ -403,8 +403,8 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster_t(FieldTArgs a)
     cy[i] = ld_cluster(rowsy + off, owner);
   }
   __syncthreads();
-  const double2 *gxh = line_dft<POW2>(cx, cxt, nq, ny, twy, false);
-  const double2 *gyh = line_dft<POW2>(cy, cyt, nq, ny, twy, false);
+  const double2 *gxh = line_dft<true>(cx, cxt, nq, ny, twy, false);
+  const double2 *gyh = line_dft<true>(cy, cyt, nq, ny, twy, false);
   // lam_hat of the own columns into a buffer neither spectrum occupies.
   double2 *lam = gxh == cx ? cxt : cx;
   double2 *lamt = gyh == cy ? cyt : cy;
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster_t(FieldTArgs a)
                           (p.x * g1.y - p.y * g1.x + r.x * g2.y - r.y * g2.x) * a.norm);
   }
   __syncthreads();
-  const double2 *cols = line_dft<POW2>(lam, lamt, nq, ny, twy, true);
+  const double2 *cols = line_dft<true>(lam, lamt, nq, ny, twy, true);
   cluster_barrier();
   for (int i = threadIdx.x; i < nr * nxh; i += blockDim.x) {
     const int r = i / nxh, kx = i - r * nxh;
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_cluster_t(FieldTArgs a)
     rx[(size_t)r * nx + kx] = make_double2(v.x, -v.y);
   }
   __syncthreads();
-  const double2 *out = line_dft<POW2>(rx, rxt, nr, nx, twx, true);
+  const double2 *out = line_dft<true>(rx, rxt, nr, nx, twx, true);
   for (int i = threadIdx.x; i < nr * nx; i += blockDim.x) a.lam[(size_t)iy0 * nx + i] = out[i].x;
   cluster_barrier();
 }
@@ -476,11 +476,11 @@ bool cluster_fits(int nx, int ny) {
   return true;
 }
 
-template <int C, bool POW2>
+template <int C>
 bool cluster_t_fits(int nx, int ny) {
   const size_t smem = field_t_bytes(nx, ny, C);
-  if (cudaFuncSetAttribute(k_field_cluster_t<C, POW2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      (C > 8 && cudaFuncSetAttribute(k_field_cluster_t<C, POW2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+  if (cudaFuncSetAttribute(k_field_cluster_t<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      (C > 8 && cudaFuncSetAttribute(k_field_cluster_t<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
                     cudaSuccess)) {
     cudaGetLastError();
     return false;
@@ -489,7 +489,7 @@ bool cluster_t_fits(int nx, int ny) {
   cudaLaunchConfig_t cfg = field_config(nx, ny, C, attr, 0);
   cfg.dynamicSmemBytes = smem;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, k_field_cluster_t<C, POW2>, &cfg) != cudaSuccess || clusters < 1) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, k_field_cluster_t<C>, &cfg) != cudaSuccess || clusters < 1) {
     cudaGetLastError();
     return false;
   }
@@ -526,9 +526,12 @@ bool field_cluster_t_available(vlp4d_ctx *c) {
   if (!field_cluster_available(c)) return false;
   if (c->field_cluster_t >= 0) return c->field_cluster_t > 0;
   c->field_cluster_t = 0;
-  const int nx = c->g.n[0], ny = c->g.n[1], C = c->field_cluster;
-  if (!(pow2_plane(nx, ny) ? (C == 16 ? cluster_t_fits<16, true>(nx, ny) : cluster_t_fits<8, true>(nx, ny))
-                           : (C == 16 ? cluster_t_fits<16, false>(nx, ny) : cluster_t_fits<8, false>(nx, ny))))
+  const int nx = c->g.n[0], ny = c->g.n[1];
+  // Powers of two only: the reverse sweeps run as graphs, in which cuFFT's kernels
+  // follow one another without launch gaps (backward over eight stored steps, us,
+  // the general transforms in one launch / cuFFT: 24 x 21 x 16 x 18 FP32 327 / 290, 25 x 12
+  // x 24 x 14 342 / 307; 16 x 32, one launch of radix-4 passes, 340 / 366).
+  if (!pow2_plane(nx, ny) || !(c->field_cluster == 16 ? cluster_t_fits<16>(nx, ny) : cluster_t_fits<8>(nx, ny)))
     return false;
   c->field_cluster_t = 1;
   return true;
@@ -549,11 +552,8 @@ int launch_field_transpose_cluster(vlp4d_ctx *c, const double *gex, const double
   cudaLaunchAttribute attr[2] = {};
   cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, attr, s);
   cfg.dynamicSmemBytes = field_t_bytes(nx, ny, c->field_cluster);
-  const bool p2 = pow2_plane(nx, ny);
-  if (c->field_cluster == 16)
-    VLP4D_CUDA_TRY(cudaLaunchKernelEx(&cfg, p2 ? k_field_cluster_t<16, true> : k_field_cluster_t<16, false>, a));
-  else
-    VLP4D_CUDA_TRY(cudaLaunchKernelEx(&cfg, p2 ? k_field_cluster_t<8, true> : k_field_cluster_t<8, false>, a));
+  if (c->field_cluster == 16) VLP4D_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_field_cluster_t<16>, a));
+  else VLP4D_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_field_cluster_t<8>, a));
   return VLP4D_OK;
 }
 
