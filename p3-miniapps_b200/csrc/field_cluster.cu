@@ -440,7 +440,8 @@ namespace {
 
 bool pow2_plane(int nx, int ny) { return (nx & (nx - 1)) == 0 && (ny & (ny - 1)) == 0; }
 
-cudaLaunchConfig_t field_config(int nx, int ny, int ctas, cudaLaunchAttribute *attr, cudaStream_t s) {
+// dep: a dependent launch, by launch_dep's rule.
+cudaLaunchConfig_t field_config(int nx, int ny, int ctas, bool dep, cudaLaunchAttribute *attr, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kFieldThreads);
@@ -453,7 +454,7 @@ cudaLaunchConfig_t field_config(int nx, int ny, int ctas, cudaLaunchAttribute *a
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = dep ? 2 : 1;
   return cfg;
 }
 
@@ -467,7 +468,7 @@ bool cluster_fits(int nx, int ny) {
     return false;
   }
   cudaLaunchAttribute attr[2] = {};
-  const cudaLaunchConfig_t cfg = field_config(nx, ny, C, attr, 0);
+  const cudaLaunchConfig_t cfg = field_config(nx, ny, C, false, attr, 0);
   int clusters = 0;
   if (cudaOccupancyMaxActiveClusters(&clusters, k_field_cluster<C, POW2>, &cfg) != cudaSuccess || clusters < 1) {
     cudaGetLastError();
@@ -486,7 +487,7 @@ bool cluster_t_fits(int nx, int ny) {
     return false;
   }
   cudaLaunchAttribute attr[2] = {};
-  cudaLaunchConfig_t cfg = field_config(nx, ny, C, attr, 0);
+  cudaLaunchConfig_t cfg = field_config(nx, ny, C, false, attr, 0);
   cfg.dynamicSmemBytes = smem;
   int clusters = 0;
   if (cudaOccupancyMaxActiveClusters(&clusters, k_field_cluster_t<C>, &cfg) != cudaSuccess || clusters < 1) {
@@ -550,7 +551,7 @@ int launch_field_transpose_cluster(vlp4d_ctx *c, const double *gex, const double
   a.ny = ny;
   a.norm = 1.0 / ((double)nx * ny);
   cudaLaunchAttribute attr[2] = {};
-  cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, attr, s);
+  cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, short_passes(c), attr, s);
   cfg.dynamicSmemBytes = field_t_bytes(nx, ny, c->field_cluster);
   if (c->field_cluster == 16) VLP4D_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_field_cluster_t<16>, a));
   else VLP4D_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_field_cluster_t<8>, a));
@@ -569,7 +570,7 @@ int launch_field_cluster(vlp4d_ctx *c, double offset, cudaStream_t s) {
   a.ky0 = 2 * M_PI / c->g.maxp[1];
   a.normcoeff = 1.0 / (double)(nx * ny);
   cudaLaunchAttribute attr[2] = {};
-  cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, attr, s);
+  cudaLaunchConfig_t cfg = field_config(nx, ny, c->field_cluster, short_passes(c), attr, s);
   const bool p2 = pow2_plane(nx, ny);
   if (c->field_cluster == 16)
     VLP4D_CUDA_TRY(cudaLaunchKernelEx(&cfg, p2 ? k_field_cluster<16, true> : k_field_cluster<16, false>, a));
