@@ -71,7 +71,6 @@ constexpr int kColsWidth = 128;   // most columns of a tile
 template <typename T, int TX, int TY, int RM, bool RHO>
 __global__ void __launch_bounds__(kColsThreads, 2) k_xy_cols(XyCols a) {
   pdl_wait();
-  pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(16) unsigned char csm[];
   T *tile = reinterpret_cast<T *>(csm);
@@ -206,7 +205,6 @@ template <typename T, bool DVX, bool DVY, int V>
 __global__ void __launch_bounds__(kVColsThreads, 4) k_v_cols(VCols a) {
   pdl_wait();
   pdl_trigger();
-  pdl_trigger();
   const unsigned gid = blockIdx.x * kVColsThreads + threadIdx.x;
   if (gid >= (unsigned)a.nxy * (unsigned)a.ngx) return;
   const int col = (int)(gid % (unsigned)a.nxy), ivx0 = (int)(gid / (unsigned)a.nxy) * V;
@@ -326,8 +324,10 @@ int run_xy_cols_rm(vlp4d_ctx *c, XyCols &a, cudaStream_t s) {
 
 template <typename T>
 int dispatch_xy_cols(vlp4d_ctx *c, XyCols &a, int tx, int ty, bool rho, cudaStream_t s) {
-  if (tx == 11 && ty == 11)
-    return rho ? run_xy_cols_rm<T, 11, 11, true>(c, a, s) : run_xy_cols_rm<T, 11, 11, false>(c, a, s);
+  if (tx == 11) {  // the FP32 time loop's joined half steps
+    if constexpr (sizeof(T) == 4) return run_xy_cols_rm<T, 11, 11, true>(c, a, s);
+    else return VLP4D_ERR_UNSUPPORTED;
+  }
   if (tx && ty) return rho ? run_xy_cols_rm<T, 6, 6, true>(c, a, s) : run_xy_cols_rm<T, 6, 6, false>(c, a, s);
   if (tx) return run_xy_cols_rm<T, 6, 0, false>(c, a, s);
   return run_xy_cols_rm<T, 0, 6, false>(c, a, s);
@@ -375,7 +375,7 @@ bool xy_cols_pay(const vlp4d_ctx *c, bool x, bool y, bool with_rho) {
 
 int launch_xy_cols(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTable *tx, const StencilTable *ty, int taps,
                    bool with_rho, cudaStream_t s) {
-  if (!c->fused || (!tx && !ty) || (taps == 11 && !(tx && ty)) || (with_rho && !(tx && ty)) ||
+  if (!c->fused || (!tx && !ty) || (taps == 11 && (!with_rho || c->dtype != VLP4D_F32)) || (with_rho && !(tx && ty)) ||
       !xy_cols_pay(c, tx, ty, with_rho))
     return VLP4D_ERR_UNSUPPORTED;
   XyCols a;

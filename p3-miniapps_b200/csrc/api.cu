@@ -418,8 +418,8 @@ static int advect_xy_impl(vlp4d_ctx *ctx, const void *fn, void *fnp1, double dt,
   rc = launch_advect_xy(ctx, fn, fnp1, tx, ty, true, true, with_rho, s);
   if (rc != VLP4D_ERR_UNSUPPORTED) return rc;
   if ((rc = fused_declined(ctx))) return rc;
-  rc = launch_xy_cols(ctx, fn, fnp1, tx, ty, 6, with_rho, s);
-  if (rc != VLP4D_ERR_UNSUPPORTED) return rc;
+  // (Without the moment launch_advect_pair_generic asks for the columns.)
+  if (with_rho && (rc = launch_xy_cols(ctx, fn, fnp1, tx, ty, 6, true, s)) != VLP4D_ERR_UNSUPPORTED) return rc;
   if ((rc = launch_advect_pair_generic(ctx, false, fn, fnp1, tx, ty, s))) return rc;
   return with_rho ? launch_field_rho(ctx, fnp1, s) : VLP4D_OK;
 }

@@ -96,8 +96,8 @@ __device__ __forceinline__ void kahan_add(double &sum, double &c, double x) {
   sum = t;
 }
 
-__global__ void k_diags(const double *rho, const double *ex, const double *ey,
-                        long long n, double dx, double dy, double *nrj_hist, double *mass_hist, double *nrjx_hist, double *nrjy_hist, int iter) {
+__global__ void k_diags(const double *rho, const double *ex, const double *ey, long long n, double dx, double dy,
+                        double *nrj_hist, double *mass_hist, double *nrjx_hist, double *nrjy_hist, int iter) {
   pdl_wait();
   // Kahan sums of rho, Ex^2 + Ey^2, Ex^2, Ey^2.
   // Each thread's elements in order; the loads of four of them are issued

@@ -318,8 +318,8 @@ bool xyxy64_available(const vlp4d_ctx *c);
 int launch_advect_xyxy_tables(vlp4d_ctx *c, const void *fn, void *fnp1, const StencilTable *x11,
                               const StencilTable *y11, bool with_rho, cudaStream_t s);
 
-// advect_cols.cu: x/y (6-tap lines, or the composed 11-tap ones with taps =
-// 11; the moment of the result into rho when with_rho) and vx/vy sweeps of
+// advect_cols.cu: x/y (6-tap lines, or in FP32 with the moment the composed 11-tap
+// ones, taps = 11; the moment of the result into rho when with_rho) and vx/vy sweeps of
 // any shape and alignment.  VLP4D_ERR_UNSUPPORTED (nothing launched) under
 // VLP4D_KERNELS=generic, for index ranges beyond 32 bits and where one thread
 // per output is faster (xy_cols_pay).
