@@ -384,7 +384,8 @@ int build_v_tables(vlp4d_ctx *c, double dt, bool vx, bool vy, cudaStream_t s) {
 int launch_advect_generic(vlp4d_ctx *c, int dim, const void *fn, void *fnp1, const StencilTable *t,
                           cudaStream_t s) {
   // By columns where that runs (45 x 39 x 51 x 43 FP64, x and y: 25 us against
-  // 76, vx and vy: 15 against 114); one thread per output under VLP4D_KERNELS=generic and beyond 32-bit indexes.
+  // 76, vx and vy: 15 against 114); one thread per output on narrow planes
+  // (xy_cols_pay), under VLP4D_KERNELS=generic and beyond 32-bit indexes.
   const int rc = dim < 2 ? launch_xy_cols(c, fn, fnp1, dim == 0 ? t : nullptr, dim == 1 ? t : nullptr, 6, false, s)
                          : launch_v_cols(c, fn, fnp1, dim == 2 ? t : nullptr, dim == 3 ? t : nullptr, s);
   if (rc != VLP4D_ERR_UNSUPPORTED) return rc;
